@@ -286,6 +286,7 @@ gf_status launch_dispatch(gf_ctx* ctx, int scatter, const AsmTables* d_tab, TC* 
 
 }  // namespace
 
+gf_status gf_assemble_node(gf_ctx* ctx, int dtype, const AsmTables* d_tab);
 gf_status gf_assemble_owner(gf_ctx* ctx, int dtype, const AsmTables* d_tab);
 gf_status gf_assemble_tc(gf_ctx* ctx, int scatter, const AsmTables* d_tab, float* K, int* d_err);
 gf_status gf_assemble_owner_gram(gf_ctx* ctx, const float* gram, float* K);
@@ -353,7 +354,8 @@ gf_status gf_assemble_launch(gf_ctx* ctx, int dtype, int scatter, int engine) {
     if (st == GF_OK) st = gf_assemble_owner_gram(ctx, ctx->d_gram, ctx->d_K32);
   } else if (scatter == GF_SCATTER_OWNER) {
     // owner-computes: every K entry (padding included) is written exactly once
-    st = gf_assemble_owner(ctx, dtype, d_tab);
+    st = gf_assemble_node_fits(ctx, dtype) ? gf_assemble_node(ctx, dtype, d_tab)
+                                           : gf_assemble_owner(ctx, dtype, d_tab);
   } else if (dtype == GF_F64) {
     cudaMemsetAsync(ctx->d_K64, 0, sizeof(double) * total, ctx->stream);
     st = launch_dispatch<double>(ctx, scatter, d_tab, ctx->d_K64);

@@ -288,14 +288,18 @@ gf_status gf_cuda_fail(gf_ctx* ctx, cudaError_t e, const char* where);
     if (e__ != cudaSuccess) return gf_cuda_fail(ctx, e__, name);      \
   } while (0)
 
+// cudaMalloc; when memory is short, the context's unused pool blocks are freed and the
+// allocation is tried once more.
+cudaError_t gf_malloc_retry(gf_ctx* ctx, void** p, size_t bytes);
+
 template <typename T>
 gf_status gf_alloc(gf_ctx* ctx, T** p, size_t count) {
   if (*p) { cudaFree(*p); *p = nullptr; }
   if (count == 0) count = 1;
-  cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
+  void* q = nullptr;
+  cudaError_t e = gf_malloc_retry(ctx, &q, count * sizeof(T));
+  *p = static_cast<T*>(q);
   if (e != cudaSuccess) {
-    cudaGetLastError();
-    *p = nullptr;
     return gf_fail(ctx, e == cudaErrorMemoryAllocation ? GF_ERR_OOM : GF_ERR_CUDA,
                    "cudaMalloc of %zu bytes failed: %s", count * sizeof(T),
                    cudaGetErrorString(e));
@@ -370,6 +374,8 @@ inline int gf_blocks(int64_t work, int threads) {
 gf_status gf_pattern_build(gf_ctx* ctx);
 gf_status gf_slotmap_ensure(gf_ctx* ctx);
 gf_status gf_color_build(gf_ctx* ctx, const int32_t* user_colors);
+bool gf_assemble_node_fits(const gf_ctx* ctx, int dtype);
+gf_status gf_geo_buffer(gf_ctx* ctx, size_t bytes);
 gf_status gf_assemble_launch(gf_ctx* ctx, int dtype, int scatter, int engine);
 gf_status gf_constraints_apply(gf_ctx* ctx, int mode);
 gf_status gf_spmv_launch(gf_ctx* ctx, int dtype, const void* x, void* y);
