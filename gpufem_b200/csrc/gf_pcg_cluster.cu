@@ -1,0 +1,318 @@
+// (P)CG for systems whose iterations are bound by launches and latency rather than by the
+// matrix: one thread-block cluster runs them all in one kernel.  Same recurrences and stopping
+// rule as the three-kernel loop in gf_solve.cu (SPRmatrix::CPU_CG,
+// src/SPRmatrix/SPRmatrix.cc:405-480).
+//
+// A CTA holds its slices of the matrix (node-block slices, gf_sell.cu) in shared memory for the
+// whole solve.  A slice's 32 nodes are a warp, each lane with its rows of r and p in registers;
+// where slices are few, further warps take a share of the slice's neighbours in the product.
+// The direction p lives in the CTAs' shared memory, a range of nodes to a CTA, and is gathered
+// from there.  An iteration has three cluster barriers: p.q, then (r.z, r.r), then the new p.
+// A CTA stores its part of a sum to every CTA before the barrier and each adds all parts after
+// it, in the same order everywhere, so a solve is reproducible.
+//
+// Microseconds per iteration (FP64 Jacobi-PCG, the three-kernel loop in brackets): Q4 64 x 64
+// 3.7 (9.8), Q8 20 x 20 3.9 (9.9), Brick8 6^3 5.9 (15.4), Brick20 4^3 8.1 (22.2).  What is left is
+// latency: a cluster barrier is 0.2 us, a sum with its barrier about 0.6.  The matrix has to fit
+// the 16 CTAs' shared memory (3.4 MB with the vectors): read from L2 instead, 16 SMs took 22.6 us
+// on Q8 64 x 64, where the loop takes 10.4 on all of them, and a grid-wide version (148 CTAs,
+// sums through global memory) took 13.
+#include <algorithm>
+
+#include "gf_internal.cuh"
+
+namespace {
+
+constexpr int kCluster = 16;          // CTAs (a size beyond 8 is opt-in)
+constexpr int kThreadsMax = 1024;
+constexpr size_t kSmemMax = 220 * 1024;   // per CTA: one to an SM
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Address of this CTA's shared address `a` in CTA `rank`
+__device__ __forceinline__ uint32_t map_rank(uint32_t a, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ double ld_cluster(uint32_t a, double) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_cluster(uint32_t a, float) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+template <int DIM, typename V>
+__device__ __forceinline__ void ld_node(uint32_t a, V (&v)[DIM]) {
+  if constexpr (DIM == 2 && sizeof(V) == 8) {
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(a) : "memory");
+  } else if constexpr (DIM == 2) {
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "r"(a) : "memory");
+  } else {
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) v[c] = ld_cluster(a + c * (uint32_t)sizeof(V), V(0));
+  }
+}
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Sums N values (of the first S warps) over the cluster; `part` is this CTA's [N][kCluster].
+template <int N>
+__device__ __forceinline__ void cluster_sum(double (&v)[N], int S, double* sh, double* part,
+                                            uint32_t part_addr) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < S) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const double s = warp_sum(v[k]);
+      if (lane == 0) sh[k * 32 + warp] = s;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      const double s = warp_sum(lane < S ? sh[k * 32 + lane] : 0.0);
+      if (lane < kCluster) st_cluster(map_rank(part_addr + (k * kCluster + cluster_rank()) * 8, lane), s);
+    }
+  }
+  cluster_sync();
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    double s = part[k * kCluster + (lane & (kCluster - 1))];
+#pragma unroll
+    for (int o = kCluster / 2; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    v[k] = s;
+  }
+}
+
+struct ClusterArgs {
+  int nnodes, S, H, iters, jacobi;   // S slices per CTA, H warps per slice
+  const int32_t* __restrict__ perm;
+  const int32_t* __restrict__ width;
+  const int64_t* __restrict__ off;
+  const int32_t* __restrict__ col;
+  SolveScalars* sc;
+};
+
+// Shared memory besides the slices: sums, directions, x and 1 / diagonal, partial products.
+template <int DIM, typename V>
+__host__ __device__ constexpr size_t cluster_vectors(int S, int H) {
+  return sizeof(double) * (3 * kCluster + 64) + sizeof(V) * DIM * 32 * (size_t)S * (2 + H);
+}
+
+template <int DIM, typename V>
+__global__ void __launch_bounds__(kThreadsMax)
+k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ dinv,
+              V* __restrict__ x, V* __restrict__ r, V* __restrict__ p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  SolveScalars* sc = A.sc;
+  if (sc->done) return;   // the same for every CTA, before any barrier
+  const int S = A.S, H = A.H, per = 32 * S;
+  double* partA = reinterpret_cast<double*>(smem_raw);       // [1][kCluster]
+  double* partB = partA + kCluster;                          // [2][kCluster]
+  double* sh = partB + 2 * kCluster;                         // [2][32]
+  V* sp = reinterpret_cast<V*>(sh + 64);                     // [per][DIM] directions of this CTA's nodes
+  V* sx = sp + (size_t)per * DIM;                            // [DIM][per] this CTA's slots
+  V* sd = sx + (size_t)per * DIM;                            // [DIM][per]
+  V* sq = sd + (size_t)per * DIM;                            // [H - 1][DIM][per]
+  V* sv = sq + (size_t)per * DIM * (H - 1);                  // the CTA's slices: values, then
+  const uint32_t sp_addr = (uint32_t)__cvta_generic_to_shared(sp);
+  const uint32_t pa = (uint32_t)__cvta_generic_to_shared(partA), pb = (uint32_t)__cvta_generic_to_shared(partB);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ks = warp % S, h = warp / S;                     // slice of the CTA, share of it
+  const int nslice = (A.nnodes + 31) >> 5;
+  const int k0 = min(nslice, (int)blockIdx.x * S), k1 = min(nslice, k0 + S);
+  const int64_t o0 = A.off[k0], cnt = A.off[k1] - o0;
+  uint32_t* sa = reinterpret_cast<uint32_t*>(sv + cnt * (DIM * DIM));   // addresses of the columns' p
+  auto home = [&](int b) {   // address of node b's direction
+    return map_rank(sp_addr + (uint32_t)((b % per) * DIM * sizeof(V)), (uint32_t)(b / per));
+  };
+  for (int64_t i = threadIdx.x; i < cnt * (DIM * DIM); i += blockDim.x) sv[i] = val[o0 * (DIM * DIM) + i];
+  for (int64_t i = threadIdx.x; i < cnt; i += blockDim.x) sa[i] = home(A.col[o0 + i]);
+  int w = 0;
+  const V* vp = sv + lane;
+  const uint32_t* ap = sa + lane;
+  if (k0 + ks < k1) {
+    w = A.width[k0 + ks];
+    const int64_t o = A.off[k0 + ks] - o0;
+    vp += o * (DIM * DIM);
+    ap += o;
+  }
+  const int li = ks * 32 + lane, slot = k0 * 32 + li;
+  const bool on = h == 0 && k0 + ks < k1 && slot < A.nnodes;
+  const int a = on ? A.perm[slot] : 0;
+  const uint32_t mine = home(a);
+  V rv[DIM], pv[DIM];
+#pragma unroll
+  for (int c = 0; c < DIM; ++c) {
+    const int64_t i = (int64_t)a * DIM + c;
+    rv[c] = on ? r[i] : V(0);
+    pv[c] = on ? p[i] : V(0);
+    if (h == 0) {
+      sx[c * per + li] = on ? x[i] : V(0);
+      sd[c * per + li] = on ? (A.jacobi ? dinv[i] : V(1)) : V(0);
+    }
+    if (on) st_cluster(mine + c * (uint32_t)sizeof(V), pv[c]);
+  }
+  double rz = sc->rzn, rr = sc->rr;
+  const double tol2 = sc->tol2;
+  int iter = sc->iter, done = 0;
+  const int maxit = sc->maxit;
+  cluster_sync();
+  for (int step = 0; step < A.iters && !done; ++step) {
+    V q[DIM];
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) q[c] = V(0);
+#pragma unroll 4
+    for (int s = h; s < w; s += H) {
+      V g[DIM];
+      ld_node<DIM, V>(ap[32 * s], g);
+      const V* e = vp + s * (DIM * DIM * 32);
+#pragma unroll
+      for (int c = 0; c < DIM; ++c)
+#pragma unroll
+        for (int c2 = 0; c2 < DIM; ++c2) q[c] += e[(c * DIM + c2) * 32] * g[c2];
+    }
+    if (H > 1) {
+      if (h > 0)
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) sq[((h - 1) * DIM + c) * per + li] = q[c];
+      __syncthreads();
+      if (h == 0)
+        for (int m = 0; m < H - 1; ++m)
+#pragma unroll
+          for (int c = 0; c < DIM; ++c) q[c] += sq[(m * DIM + c) * per + li];
+    }
+    double sum[1] = {0.0};
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) sum[0] += (double)pv[c] * (double)q[c];
+    cluster_sum<1>(sum, S, sh, partA, pa);
+    const double pq = sum[0];
+    if (!(pq > 0.0) || !isfinite(pq)) {
+      done = 2;
+      break;
+    }
+    const V alpha = (V)(rz / pq);
+    double two[2] = {0.0, 0.0};
+    V zv[DIM];
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      zv[c] = V(0);
+      if (h == 0) {
+        sx[c * per + li] = fma(alpha, pv[c], sx[c * per + li]);
+        rv[c] = fma(-alpha, q[c], rv[c]);
+        zv[c] = rv[c] * sd[c * per + li];
+        two[0] += (double)rv[c] * (double)zv[c];
+        two[1] += (double)rv[c] * (double)rv[c];
+      }
+    }
+    cluster_sum<2>(two, S, sh, partB, pb);
+    const V beta = (V)(two[0] / rz);
+    rz = two[0];
+    rr = two[1];
+    ++iter;
+    if (rr <= tol2) done = 1;
+    else if (iter >= maxit) done = 3;
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      pv[c] = fma(beta, pv[c], zv[c]);
+      if (on) st_cluster(mine + c * (uint32_t)sizeof(V), pv[c]);
+    }
+    cluster_sync();
+  }
+  cluster_sync();   // no CTA leaves while another may still write to it
+  if (on)
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      const int64_t i = (int64_t)a * DIM + c;
+      x[i] = sx[c * per + li];
+      r[i] = rv[c];
+      p[i] = pv[c];
+    }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc->rzn = rz;
+    sc->rr = rr;
+    sc->iter = iter;
+    sc->done = done;
+  }
+}
+
+template <int DIM, typename V>
+gf_status run_cluster(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V* p, int iters, int* ran) {
+  *ran = 0;
+  const int nslice = (ctx->nnodes + 31) / 32;
+  const int S = (nslice + kCluster - 1) / kCluster;
+  if (S > kThreadsMax / 32) return GF_OK;
+  // a CTA's slices at the widest row
+  const size_t slices = (size_t)S * 32 * (ctx->W / DIM) * (DIM * DIM * sizeof(V) + 4);
+  int H = 1;
+  while (S * H * 2 <= 16 && cluster_vectors<DIM, V>(S, H * 2) + slices <= kSmemMax) H *= 2;
+  const size_t sm = cluster_vectors<DIM, V>(S, H) + slices;
+  if (sm > kSmemMax) return GF_OK;
+  auto kern = k_pcg_cluster<DIM, V>;
+  GF_CUDA(ctx, gf_smem_attr(kern, sm));
+  GF_CUDA(ctx, gf_func_attr((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  ClusterArgs A{ctx->nnodes, S, H, iters, dinv != nullptr, ctx->d_sell_perm, ctx->d_sell_w,
+                ctx->d_sell_off, ctx->d_sell_col, ctx->d_scal};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kCluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kCluster);
+  cfg.blockDim = dim3(S * H * 32);
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = ctx->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, A, val, dinv, x, r, p) != cudaSuccess) {
+    cudaGetLastError();   // no room for such a cluster here: nothing was done
+    return GF_OK;
+  }
+  ctx->launches++;
+  GF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, ctx->d_scal, sizeof(SolveScalars), cudaMemcpyDeviceToHost,
+                               ctx->stream));
+  GF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  *ran = 1;
+  return GF_OK;
+}
+
+}  // namespace
+
+// Runs up to `iters` iterations of the (P)CG whose state is in x, r, p and the context's scalars
+// (iter, rr, rzn, done updated and read back to the pinned copy).  *ran = 0: the system is not
+// one for this kernel, and nothing was done.  dinv = null: no preconditioner.
+gf_status gf_pcg_cluster(gf_ctx* ctx, const double* val, const double* dinv, double* x, double* r,
+                         double* p, int iters, int* ran) {
+  *ran = 0;
+  if (ctx->sell_bdim == 2) return run_cluster<2, double>(ctx, val, dinv, x, r, p, iters, ran);
+  if (ctx->sell_bdim == 3) return run_cluster<3, double>(ctx, val, dinv, x, r, p, iters, ran);
+  return GF_OK;
+}
+gf_status gf_pcg_cluster(gf_ctx* ctx, const float* val, const float* dinv, float* x, float* r,
+                         float* p, int iters, int* ran) {
+  *ran = 0;
+  if (ctx->sell_bdim == 2) return run_cluster<2, float>(ctx, val, dinv, x, r, p, iters, ran);
+  if (ctx->sell_bdim == 3) return run_cluster<3, float>(ctx, val, dinv, x, r, p, iters, ran);
+  return GF_OK;
+}

@@ -665,6 +665,23 @@ gf_status run_cg(gf_ctx* ctx, MatLayout L, const TK* val, const V* b, CgVecs vv,
   GF_LAUNCH_CHECK(ctx, "k_cg_init");
   k_cg_init_fin<<<1, 1, 0, s>>>(sc, eps, maxit);
   GF_LAUNCH_CHECK(ctx, "k_cg_init_fin");
+  SolveScalars* hs = (SolveScalars*)ctx->h_pinned;
+  // small systems: every iteration in one kernel (with a time limit, a launch per check_every
+  // iterations)
+  for (;;) {
+    int ran = 0;
+    gf_status st = gf_pcg_cluster(ctx, val, dinv, x, r, p, max_seconds > 0.0 ? check_every : maxit, &ran);
+    if (st != GF_OK) return st;
+    if (!ran) break;
+    if (!hs->done && max_seconds > 0.0 &&
+        std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() <= max_seconds)
+      continue;
+    *iters = hs->iter;
+    *done_code = hs->done;
+    *rr_final = hs->rr;
+    *rr0_out = hs->rr0;
+    return GF_OK;
+  }
 
   // capture one chunk of iterations as a graph
   cudaGraph_t graph = nullptr;
@@ -682,7 +699,6 @@ gf_status run_cg(gf_ctx* ctx, MatLayout L, const TK* val, const V* b, CgVecs vv,
     cudaGraphDestroy(graph);
     return gf_cuda_fail(ctx, ce, "graph instantiate");
   }
-  SolveScalars* hs = (SolveScalars*)ctx->h_pinned;
   gf_status st = GF_OK;
   for (;;) {
     ce = cudaGraphLaunch(exec, s);
