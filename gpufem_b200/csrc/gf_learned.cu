@@ -85,6 +85,7 @@ struct LpState {
   double* dinv64 = nullptr;
   float* dlog = nullptr;     // log(d / mean d)
   float* dvec = nullptr;     // d (loss weight)
+  double* logsum = nullptr;  // block sums of log d
   // activations [N][H] (pre-activations kept for the ReLU masks)
   float* feat = nullptr;     // [N][4 dim]
   float* v1 = nullptr;       // [n] D^-1 K rho
@@ -107,7 +108,9 @@ struct LpState {
   float* pr = nullptr;       // [npairs][n]
   float* pe = nullptr;       // [npairs][n]
   int* err = nullptr;        // set by a tensor-core layer whose MMA wait timed out
-  bool ready = false;        // diag / graph set up for the current matrix
+  bool ready = false;        // diag / graph set up for version `ver` of K64 (ver64) or K32
+  bool ver64 = false;
+  int64_t ver = -1;
   bool coarse = false;       // with the two-level coarse correction (gf_lp_set_coarse)
   int loss = GF_LP_LOSS_ERROR;
 };
@@ -660,27 +663,52 @@ __global__ void k_lp_degree(int N, const int32_t* __restrict__ adj_off, float* _
   if (a < N) deg_inv[a] = 1.f / (float)max(1, adj_off[a + 1] - adj_off[a]);
 }
 
-// diagonal of K: d, 1/d (FP32 and FP64) and log(d / mean d) (mean taken on the host)
-template <typename TK>
-__global__ void k_lp_diag(int n, const int32_t* __restrict__ rownnz, const int32_t* __restrict__ col,
-                          const TK* __restrict__ val, float* __restrict__ d,
-                          float* __restrict__ dinv, double* __restrict__ dinv64) {
-  const int row = blockIdx.x * kLT + threadIdx.x;
-  if (row >= n) return;
-  double dv = 0.0;
-  for (int s = 0; s < rownnz[row]; ++s) {
-    const int64_t o = (int64_t)s * n + row;
-    if (col[o] == row) { dv = (double)val[o]; break; }
-  }
-  if (!(dv > 0.0)) dv = 1.0;
-  d[row] = (float)dv;
-  dinv[row] = (float)(1.0 / dv);
-  dinv64[row] = 1.0 / dv;
+// Sum over the block (kLT threads), the same in every thread.
+__device__ inline double lp_block_total(double v, double* sh /* [kLT / 32] */) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double s = 0.0;
+#pragma unroll
+  for (int w = 0; w < kLT / 32; ++w) s += sh[w];
+  return s;
 }
 
-__global__ void k_lp_dlog(int n, const float* __restrict__ d, double logmean, float* __restrict__ dlog) {
-  const int i = blockIdx.x * kLT + threadIdx.x;
-  if (i < n) dlog[i] = (float)(log((double)d[i]) - logmean);
+// Diagonal of K (at every node's own slot): d, 1/d (FP32 and FP64), and the block's sum of
+// log d for k_lp_dlog.
+constexpr int kLpDiagCtas = 148 * 4;
+template <typename TK>
+__global__ void __launch_bounds__(kLT)
+k_lp_diag(int n, int dim, const int32_t* __restrict__ diagpos, const TK* __restrict__ val,
+          float* __restrict__ d, float* __restrict__ dinv, double* __restrict__ dinv64,
+          double* __restrict__ logsum) {
+  __shared__ double sh[kLT / 32];
+  double ls = 0.0;
+  for (int row = blockIdx.x * kLT + threadIdx.x; row < n; row += gridDim.x * kLT) {
+    const int a = row / dim, c = row - a * dim;
+    double dv = (double)val[(int64_t)(diagpos[a] * dim + c) * n + row];
+    if (!(dv > 0.0)) dv = 1.0;
+    d[row] = (float)dv;
+    dinv[row] = (float)(1.0 / dv);
+    dinv64[row] = 1.0 / dv;
+    ls += log((double)(float)dv);
+  }
+  ls = lp_block_total(ls, sh);
+  if (threadIdx.x == 0) logsum[blockIdx.x] = ls;
+}
+
+// log(d / geometric mean of d)
+__global__ void __launch_bounds__(kLT)
+k_lp_dlog(int n, int parts, const double* __restrict__ logsum, const float* __restrict__ d,
+          float* __restrict__ dlog) {
+  __shared__ double sh[kLT / 32];
+  double ls = 0.0;
+  for (int k = threadIdx.x; k < parts; k += kLT) ls += logsum[k];
+  const double mean = lp_block_total(ls, sh) / n;
+  for (int i = blockIdx.x * kLT + threadIdx.x; i < n; i += gridDim.x * kLT)
+    dlog[i] = (float)(log((double)d[i]) - mean);
 }
 
 __global__ void k_lp_cast_f32(int n, const double* __restrict__ a, float* __restrict__ b) {
@@ -704,7 +732,7 @@ static void lp_free_buffers(LpState* s) {
   f(s->v1); f(s->v2); f(s->lw); f(s->ls); f(s->lt);
   for (int l = 0; l <= kLayers; ++l) { f(s->pre[l]); f(s->h[l]); }
   for (int l = 0; l < kLayers; ++l) f(s->agg[l]);
-  f(s->y); f(s->dy); f(s->rho); f(s->dh); f(s->dpre); f(s->tmp);
+  f(s->y); f(s->dy); f(s->rho); f(s->dh); f(s->dpre); f(s->tmp); f(s->logsum);
   f(s->pr); f(s->pe);
   s->npairs = 0;
   s->ready = false;
@@ -720,7 +748,9 @@ void gf_lp_free(gf_ctx* ctx) {
   ctx->lp = nullptr;
 }
 
-// Allocates the per-mesh buffers and the diagonal / graph data for the current matrix.
+// Allocates the per-mesh buffers and the diagonal / graph data for the current matrix, once
+// per version of its values.  (Before every application instead, with the mean of log d taken
+// on the host, this was most of the call: Brick8 32^3 755 us, 211 us now.)
 gf_status gf_lp_prepare(gf_ctx* ctx) {
   LpState* s = ctx->lp;
   if (!s) return gf_fail(ctx, GF_ERR_STATE, "learned preconditioner not initialised");
@@ -728,16 +758,20 @@ gf_status gf_lp_prepare(gf_ctx* ctx) {
     return gf_fail(ctx, GF_ERR_STATE, "learned preconditioner needs an assembled mesh");
   if (s->dim != ctx->dim)
     return gf_fail(ctx, GF_ERR_STATE, "weights are for dim %d, mesh has dim %d", s->dim, ctx->dim);
+  if (!ctx->d_diagpos) return gf_fail(ctx, GF_ERR_STATE, "learned preconditioner needs a mesh-built pattern");
   const int N = ctx->nnodes, n = ctx->n, dim = ctx->dim;
-  if (s->ready && s->N == N && s->n == n) {
-    // refresh the diagonal (the matrix may have changed)
-  } else {
+  const int64_t ver = ctx->has64 ? ctx->kver64 : ctx->kver32;
+  gf_status st = gf_sell_prepare(ctx, ctx->has64 ? GF_F64 : GF_F32);  // feature products
+  if (st != GF_OK) return st;
+  if (s->ready && s->N == N && s->n == n && s->ver == ver && s->ver64 == ctx->has64)
+    return GF_OK;   // set up for these values of K (the versions only grow)
+  if (!s->ready || s->N != N || s->n != n) {
     lp_free_buffers(s);
     s->N = N;
     s->n = n;
-    gf_status st;
 #define LPA(p, cnt) if ((st = lp_alloc(ctx, &(p), (size_t)(cnt))) != GF_OK) return st
     LPA(s->deg_inv, N); LPA(s->dinv, n); LPA(s->dinv64, n); LPA(s->dlog, n); LPA(s->dvec, n);
+    LPA(s->logsum, kLpDiagCtas);
     LPA(s->feat, (size_t)N * 4 * dim);
     LPA(s->v1, n); LPA(s->v2, n); LPA(s->lw, n); LPA(s->ls, n); LPA(s->lt, n);
     for (int l = 0; l <= kLayers; ++l) { LPA(s->pre[l], (size_t)N * H); LPA(s->h[l], (size_t)N * H); }
@@ -746,30 +780,21 @@ gf_status gf_lp_prepare(gf_ctx* ctx) {
     LPA(s->tmp, (size_t)N * H);
 #undef LPA
   }
-  {
-    gf_status st = gf_sell_prepare(ctx, ctx->has64 ? GF_F64 : GF_F32);  // feature products
-    if (st != GF_OK) return st;
-  }
   cudaStream_t st_ = ctx->stream;
+  const int parts = std::min(gf_blocks(n, kLT), kLpDiagCtas);
   k_lp_degree<<<gf_blocks(N, kLT), kLT, 0, st_>>>(N, ctx->d_adj_off, s->deg_inv);
-  ctx->launches++;
   if (ctx->has64)
-    k_lp_diag<double><<<gf_blocks(n, kLT), kLT, 0, st_>>>(n, ctx->d_rownnz, ctx->d_colidx,
-                                                          ctx->d_K64, s->dvec, s->dinv, s->dinv64);
+    k_lp_diag<double><<<parts, kLT, 0, st_>>>(n, dim, ctx->d_diagpos, ctx->d_K64, s->dvec, s->dinv,
+                                              s->dinv64, s->logsum);
   else
-    k_lp_diag<float><<<gf_blocks(n, kLT), kLT, 0, st_>>>(n, ctx->d_rownnz, ctx->d_colidx,
-                                                         ctx->d_K32, s->dvec, s->dinv, s->dinv64);
-  ctx->launches++;
-  std::vector<float> d(n);
-  GF_CUDA(ctx, cudaMemcpyAsync(d.data(), s->dvec, sizeof(float) * n, cudaMemcpyDeviceToHost, st_));
-  GF_CUDA(ctx, cudaStreamSynchronize(st_));
-  double lm = 0.0;
-  for (float x : d) lm += std::log((double)x);
-  lm /= n;
-  k_lp_dlog<<<gf_blocks(n, kLT), kLT, 0, st_>>>(n, s->dvec, lm, s->dlog);
-  ctx->launches++;
+    k_lp_diag<float><<<parts, kLT, 0, st_>>>(n, dim, ctx->d_diagpos, ctx->d_K32, s->dvec, s->dinv,
+                                             s->dinv64, s->logsum);
+  k_lp_dlog<<<parts, kLT, 0, st_>>>(n, parts, s->logsum, s->dvec, s->dlog);
+  ctx->launches += 3;
   GF_CUDA(ctx, cudaGetLastError());
   s->ready = true;
+  s->ver = ver;
+  s->ver64 = ctx->has64;
   return GF_OK;
 }
 
@@ -845,7 +870,8 @@ static gf_status lp_mm_setup(gf_ctx* ctx, int dim) {
 // Timeout flag of the tensor-core layers (read after a synchronisation).
 static gf_status lp_check_err(gf_ctx* ctx) {
   int h = 0;
-  GF_CUDA(ctx, cudaMemcpy(&h, ctx->lp->err, sizeof(int), cudaMemcpyDeviceToHost));
+  GF_CUDA(ctx, cudaMemcpyAsync(&h, ctx->lp->err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  GF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (h) return gf_fail(ctx, GF_ERR_CUDA, "learned network: an MMA completion wait timed out");
   return GF_OK;
 }
@@ -1115,11 +1141,11 @@ GF_API gf_status gf_lp_apply(gf_ctx* ctx, const float* r, float* z) {
   k_lp_output<float><<<gf_blocks(s->n, kLT), kLT, 0, ctx->stream>>>(s->n, s->rho, s->y, s->sc, z);
   GF_LAUNCH_CHECK(ctx, "k_lp_output");
   cudaEventRecord(ctx->ev1, ctx->stream);
-  GF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  if ((st = lp_check_err(ctx)) != GF_OK) return st;   // waits for the stream
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
   ctx->last_seconds = ms * 1e-3;   // device time of one application (gf_last_device_seconds)
-  return lp_check_err(ctx);
+  return GF_OK;
 }
 
 // Loss and gradient for one (r, e) pair of FP32 device vectors; the gradient of
