@@ -48,7 +48,7 @@ __device__ inline double block_sum(T v, double* sh) {
 //         off[t/32] + 32 s + t%32, and every row of a slice runs to the slice's
 //         width (padding entries hold column t and value 0).
 struct MatLayout {
-  int count;  // threads to launch
+  int count;  // rows
   int n;
   const int32_t* __restrict__ rownnz;
   const int32_t* __restrict__ col;
@@ -57,7 +57,7 @@ struct MatLayout {
   int bdim = 0;      // 0: rows (ELL / SELL); 2, 3: node-block slices (gf_sell.cu)
   int nnodes = 0;
   const int32_t* __restrict__ perm = nullptr;  // node-block slices: node of each slot
-  int threads = kT;  // block size
+  int split = 1;  // node-block slices: warps that share a slice (slice_split)
 
   __device__ inline bool at(int t, int& nz, int64_t& o, int64_t& stride) const {
     if (t >= count) return false;
@@ -122,125 +122,198 @@ __device__ inline void ldg_pair(const double* __restrict__ x, int b, Acc& x0, Ac
   x1 = (Acc)v.y;
 }
 
-// Node-block slices: thread t computes the DIM rows of node perm[t] (slice k = t / 32,
-// lane l = t % 32).  Per neighbour block it reads one coalesced column word, DIM x DIM
-// coalesced values and DIM consecutive entries of x (once for all DIM rows), and it
-// writes its DIM results contiguously.  Measured against a warp per (slice, component),
-// which gathers x DIM times: Q8 512 FP64 113 -> 96 us, FP32 78 -> 60 us, Brick8 128
-// FP32 459 -> 373 us (B200, L2 flushed).
-template <int DIM, typename TK, typename TX>
-__device__ inline bool node_rows(const MatLayout& L, int t, const TK* __restrict__ val,
-                                 const TX* __restrict__ x, int& node, double (&out)[DIM]) {
-  using Acc = typename std::conditional<sizeof(TK) == 8 || sizeof(TX) == 8, double, float>::type;
-  constexpr int SS = DIM * DIM * 32;  // value stride between neighbour slots
-  if (t >= L.nnodes) return false;
-  node = __ldg(L.perm + t);
-  const int k = t >> 5, l = t & 31;
-  const int64_t o = __ldg(L.off + k);
-  const int w = __ldg(L.width + k);
-  const int32_t* bc = L.col + o + l;
-  const TK* vp = val + o * (DIM * DIM) + l;
-  Acc acc[DIM];
+// How a kernel walks the matrix: each policy calls f(row, (K x)[row]) for every row, from one
+// thread per row, and knows its block and grid.  A kernel is instantiated per policy, so that
+// the registers of one do not limit the warps in flight of another.
+
+// ELL / SELL: a thread per row, rows strided over a capped grid.
+struct RowWalk {
+  static constexpr int kThreads = kT;
+  static int grid(const gf_ctx* ctx, const MatLayout& L) {
+    return std::min(gf_blocks(L.count, kThreads), ctx->sm_count * 8);
+  }
+  template <typename TK, typename TX, typename F>
+  __device__ static void rows(const MatLayout& L, const TK* __restrict__ val,
+                              const TX* __restrict__ x, F&& f) {
+    for (int t = blockIdx.x * kThreads + threadIdx.x; t < L.count; t += gridDim.x * kThreads) {
+      int nz;
+      int64_t o, st;
+      if (L.at(t, nz, o, st)) f(t, row_dot(o, st, nz, L.col, val, x));
+    }
+  }
+};
+
+// Node-block slices: SPLIT warps share slice k (32 nodes), lane l of each works on the DIM rows
+// of node perm[32 k + l], over the neighbour slots part, part + SPLIT, ...; the partial rows
+// are added through shared memory by the first of the warps.  Per neighbour slot a thread reads
+// one coalesced column word, DIM x DIM coalesced values and DIM consecutive entries of x (once
+// for all DIM rows); UN slots are in flight at a time.
+//
+// Bound: the matrix is read once, so HBM, as long as enough warps have loads in flight.  One
+// warp per slice leaves that to the number of slices: a Brick20 row has up to 81 neighbour
+// slots, which one warp walks serially (column -> gather -> sums), and a 24^3 mesh has only 13
+// slices per SM.  Four warps per slice, one slot at a time, against one (events around the
+// call, L2 flushed): Brick20 FP64 12^3 57 -> 18 us, 24^3 67 -> 52, 48^3 342 -> 314, FP32 40^3
+// 126 -> 111.  A Brick8 row has 27 slots: four warps lose (96^3 FP32 170 -> 188), two warps
+// with two slots in flight win (165; 128^3 381 -> 372, 20^3 21.6 -> 14.7).  2-D rows are short:
+// splitting costs on large meshes (Q8 512 FP32 56 -> 65), and one warp per slice gains from the
+// registers alone (58 -> 54); where that leaves the SMs with few warps, two per slice win (Q8
+// 128 PCG FP64 13.5 -> 12.4 us an iteration, 12.9 with one and 14.7 with four).  Whole PCG
+// iterations in FP64: Brick20 14^3 38.5 -> 16.7 us, 24^3 59.4 -> 49.4, 32^3 108 -> 101, Brick8
+// 30^3 22.4 -> 16.9, 64^3 99.0 -> 98.8.
+// Eight warps per slice, four slots in flight, blocks of 64, launch bounds that force more warps
+// per SM, and a bulk prefetch of the slice into L2 all measured slower.  The bounds name one
+// block per SM: without it the compiler aims at 32 registers, which serialises a slot's loads
+// (Brick20 24^3 FP64 52 -> 71 us).
+template <int DIM, int SPLIT, int UN>
+struct NodeWalk {
+  static constexpr int kThreads = 128;
+  static constexpr int kSlices = kThreads / 32 / SPLIT;  // per block
+  static int grid(const gf_ctx*, const MatLayout& L) {
+    return gf_blocks(gf_blocks(L.nnodes, 32), kSlices);
+  }
+
+  template <int N, typename TK, typename TX, typename Acc>
+  __device__ static void slots(const int32_t* __restrict__ bc, const TK* __restrict__ vp,
+                               const TX* __restrict__ x, Acc (&acc)[DIM]) {
+    constexpr int kSlot = DIM * DIM * 32;  // value stride between neighbour slots
+    int b[N];
+    TK u[N][DIM * DIM];
+    Acc xv[N][DIM];
 #pragma unroll
-  for (int c = 0; c < DIM; ++c) acc[c] = 0;
-  if constexpr (DIM == 2) {
-    // short 2-D rows: all column words first, so every x gather's address is known
-    // before the first one is issued
-    constexpr int kPre = 24;
-    if (w <= kPre) {
-      int bb[kPre];
+    for (int i = 0; i < N; ++i) b[i] = __ldcs(bc + 32 * (i * SPLIT));
 #pragma unroll
-      for (int p = 0; p < kPre; ++p) bb[p] = p < w ? __ldcs(bc + 32 * p) : 0;
+    for (int i = 0; i < N; ++i)
 #pragma unroll
-      for (int p = 0; p < kPre; ++p) {
-        if (p < w) {
-          const TK* v = vp + p * SS;
-          const TK u0 = __ldcs(v), u1 = __ldcs(v + 32), u2 = __ldcs(v + 64), u3 = __ldcs(v + 96);
-          Acc x0, x1;
-          ldg_pair(x, bb[p], x0, x1);
-          acc[0] += (Acc)u0 * x0 + (Acc)u1 * x1;
-          acc[1] += (Acc)u2 * x0 + (Acc)u3 * x1;
+      for (int e = 0; e < DIM * DIM; ++e) u[i][e] = __ldcs(vp + i * SPLIT * kSlot + e * 32);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      if constexpr (DIM == 2) {
+        ldg_pair(x, b[i], xv[i][0], xv[i][1]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) xv[i][c] = (Acc)__ldg(x + (int64_t)b[i] * DIM + c);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        if constexpr (DIM == 2) {  // by pairs: half as many roundings on the running sum
+          acc[c] += (Acc)u[i][2 * c] * xv[i][0] + (Acc)u[i][2 * c + 1] * xv[i][1];
+        } else {
+#pragma unroll
+          for (int e = 0; e < DIM; ++e) acc[c] += (Acc)u[i][c * DIM + e] * xv[i][e];
         }
       }
-      out[0] = (double)acc[0];
-      out[1] = (double)acc[1];
-      return true;
+  }
+
+  template <typename TK, typename TX, typename F>
+  __device__ static void rows(const MatLayout& L, const TK* __restrict__ val,
+                              const TX* __restrict__ x, F&& f) {
+    using Acc =
+        typename std::conditional<sizeof(TK) == 8 || sizeof(TX) == 8, double, float>::type;
+    __shared__ Acc sh[SPLIT > 1 ? kSlices * (SPLIT - 1) * DIM * 32 : 1];
+    const int warp = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int g = warp / SPLIT, part = warp % SPLIT;
+    const int k = blockIdx.x * kSlices + g, t = k * 32 + l;
+    Acc acc[DIM];
+    if (t < L.nnodes) {
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) acc[c] = 0;
+      const int64_t o = __ldg(L.off + k);
+      const int w = __ldg(L.width + k);
+      const int32_t* bc = L.col + o + l + 32 * part;
+      const TK* vp = val + (o + 32 * part) * (DIM * DIM) + l;
+      int p = part;
+      for (; p + (UN - 1) * SPLIT < w; p += UN * SPLIT) {
+        slots<UN>(bc, vp, x, acc);
+        bc += UN * SPLIT * 32;
+        vp += UN * SPLIT * 32 * DIM * DIM;
+      }
+      if constexpr (UN > 1)
+        for (; p < w; p += SPLIT) {
+          slots<1>(bc, vp, x, acc);
+          bc += SPLIT * 32;
+          vp += SPLIT * 32 * DIM * DIM;
+        }
+      if (part) {
+#pragma unroll
+        for (int c = 0; c < DIM; ++c)
+          sh[((g * (SPLIT - 1) + part - 1) * DIM + c) * 32 + l] = acc[c];
+      }
+    }
+    if constexpr (SPLIT > 1) __syncthreads();
+    if (t < L.nnodes && part == 0) {
+      const int node = __ldg(L.perm + t);
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        double v = (double)acc[c];
+#pragma unroll
+        for (int q = 0; q < SPLIT - 1; ++q)
+          v += (double)sh[((g * (SPLIT - 1) + q) * DIM + c) * 32 + l];
+        f(node * DIM + c, v);
+      }
     }
   }
-  for (int p = 0; p < w; ++p, bc += 32, vp += SS) {
-    const int b = __ldcs(bc);
-    TK u[DIM * DIM];
-#pragma unroll
-    for (int e = 0; e < DIM * DIM; ++e) u[e] = __ldcs(vp + e * 32);
-    Acc xv[DIM];
-#pragma unroll
-    for (int c2 = 0; c2 < DIM; ++c2) xv[c2] = (Acc)__ldg(x + (int64_t)b * DIM + c2);
-#pragma unroll
-    for (int c = 0; c < DIM; ++c)
-#pragma unroll
-      for (int c2 = 0; c2 < DIM; ++c2) acc[c] += (Acc)u[c * DIM + c2] * xv[c2];
-  }
-#pragma unroll
-  for (int c = 0; c < DIM; ++c) out[c] = (double)acc[c];
-  return true;
+};
+
+// Warps per slice (measured above): 3-D by the mean number of slots of a row, between Brick8's
+// 27 and Brick20's 52; 2-D by whether a warp per slice would give an SM 16 warps.
+inline int slice_split(const gf_ctx* ctx, int dim, int nnodes, int64_t slots) {
+  const int64_t nslice = gf_blocks(nnodes, 32);
+  if (dim == 3) return slots >= 40 * nslice ? 4 : 2;
+  return nslice <= 16 * (int64_t)ctx->sm_count ? 2 : 1;
 }
 
-// Calls f(row, (K x)[row]) for every row that thread t of layout L computes.
-template <typename TK, typename TX, typename F>
-__device__ inline void mat_rows(const MatLayout& L, int t, const TK* __restrict__ val,
-                                const TX* __restrict__ x, F&& f) {
-  int a;
-  if (L.bdim == 2) {
-    double v[2];
-    if (node_rows<2>(L, t, val, x, a, v)) {
-      f(2 * a, v[0]);
-      f(2 * a + 1, v[1]);
-    }
-  } else if (L.bdim == 3) {
-    double v[3];
-    if (node_rows<3>(L, t, val, x, a, v)) {
-      f(3 * a, v[0]);
-      f(3 * a + 1, v[1]);
-      f(3 * a + 2, v[2]);
-    }
-  } else {
-    int nz;
-    int64_t o, st;
-    if (L.at(t, nz, o, st)) f(t, row_dot(o, st, nz, L.col, val, x));
-  }
+// Calls g(walk) with the policy of layout L.
+template <typename G>
+inline void with_walk(const MatLayout& L, G&& g) {
+  if (L.bdim == 2)
+    L.split == 1 ? g(NodeWalk<2, 1, 1>{}) : g(NodeWalk<2, 2, 1>{});
+  else if (L.bdim == 3)
+    L.split == 2 ? g(NodeWalk<3, 2, 2>{}) : g(NodeWalk<3, 4, 1>{});
+  else
+    g(RowWalk{});
 }
 
-template <typename TK, typename TX, typename TY>
-__global__ void __launch_bounds__(kT)
+// launches the kernel (in parentheses, a template over `Walk`) over the rows of L on stream s
+#define GF_ROWS_LAUNCH(ctx, s, L, KERNEL, ...)                                    \
+  with_walk(L, [&](auto walk) {                                                   \
+    using Walk = decltype(walk);                                                  \
+    GF_UNPAREN KERNEL<<<Walk::grid(ctx, L), Walk::kThreads, 0, s>>>(L, __VA_ARGS__); \
+  })
+#define GF_UNPAREN(...) __VA_ARGS__
+
+template <class W, typename TK, typename TX, typename TY>
+__global__ void __launch_bounds__(W::kThreads, 1)
 k_spmv(MatLayout L, const TK* __restrict__ val, const TX* __restrict__ x, TY* __restrict__ y) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < L.count; t += gridDim.x * blockDim.x)
-    mat_rows(L, t, val, x, [&](int row, double v) { y[row] = (TY)v; });
+  W::rows(L, val, x, [&](int row, double v) { y[row] = (TY)v; });
 }
 
 // y = scale .* (K x) for FP32 x and y (scale may be null), FP64 accumulation with FP64
 // values
-template <typename TK>
-__global__ void __launch_bounds__(kT)
+template <class W, typename TK>
+__global__ void __launch_bounds__(W::kThreads, 1)
 k_spmv_rowscale(MatLayout L, const TK* __restrict__ val, const float* __restrict__ x,
                 const float* __restrict__ scale, float* __restrict__ y) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < L.count; t += gridDim.x * blockDim.x)
-    mat_rows(L, t, val, x, [&](int row, double v) {
-      y[row] = (float)(scale ? v * (double)__ldg(scale + row) : v);
-    });
+  W::rows(L, val, x, [&](int row, double v) {
+    y[row] = (float)(scale ? v * (double)__ldg(scale + row) : v);
+  });
 }
 
 // r = f - K u (FP64), and r.r
-__global__ void __launch_bounds__(kT)
+template <class W>
+__global__ void __launch_bounds__(W::kThreads, 1)
 k_residual64(MatLayout L, const double* __restrict__ val, const double* __restrict__ u,
              const double* __restrict__ f, double* __restrict__ r, double* __restrict__ acc) {
   __shared__ double sh[32];
   double rr = 0.0;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < L.count; t += gridDim.x * blockDim.x)
-    mat_rows(L, t, val, u, [&](int row, double kv) {
-      const double v = f[row] - kv;
-      r[row] = v;
-      rr += v * v;
-    });
+  W::rows(L, val, u, [&](int row, double kv) {
+    const double v = f[row] - kv;
+    r[row] = v;
+    rr += v * v;
+  });
   double s = block_sum(rr, sh);
   if (threadIdx.x == 0) atomicAdd(acc, s);
 }
@@ -315,8 +388,8 @@ __global__ void k_cg_init_fin(SolveScalars* sc, double eps, int maxit) {
   sc->done = (sc->rr <= 0.0 || sc->rr <= sc->tol2) ? 1 : (maxit <= 0 ? 3 : 0);
 }
 
-template <typename TK, typename V>
-__global__ void __launch_bounds__(kT)
+template <class W, typename TK, typename V>
+__global__ void __launch_bounds__(W::kThreads, 1)
 k_cg_spmv_dot(MatLayout L, const TK* __restrict__ val, const V* __restrict__ p,
               V* __restrict__ q, SolveScalars* sc) {
   __shared__ double sh[32];
@@ -327,11 +400,10 @@ k_cg_spmv_dot(MatLayout L, const TK* __restrict__ val, const V* __restrict__ p,
     sc->rr = 0.0;
   }
   double pq = 0.0;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < L.count; t += gridDim.x * blockDim.x)
-    mat_rows(L, t, val, p, [&](int row, double v) {
-      q[row] = (V)v;
-      pq += (double)p[row] * (double)(V)v;
-    });
+  W::rows(L, val, p, [&](int row, double v) {
+    q[row] = (V)v;
+    pq += (double)p[row] * (double)(V)v;
+  });
   double s = block_sum(pq, sh);
   if (threadIdx.x == 0) atomicAdd(&sc->pq, s);
 }
@@ -344,7 +416,8 @@ __global__ void k_copy_f32(int n, const double* __restrict__ a, float* __restric
 // q = K32 p on the FP32 matrix from the FP32 copy p32 of the FP64 direction p: FP32
 // products and row sums (no FP64 conversion per matrix entry, which measured 81 against
 // 52 us on Q8 512), q and the p.q dot in FP64.
-__global__ void __launch_bounds__(kT)
+template <class W>
+__global__ void __launch_bounds__(W::kThreads, 1)
 k_cg_spmv_dot_x32(MatLayout L, const float* __restrict__ val, const float* __restrict__ p32,
                   const double* __restrict__ p, double* __restrict__ q, SolveScalars* sc) {
   __shared__ double sh[32];
@@ -355,11 +428,10 @@ k_cg_spmv_dot_x32(MatLayout L, const float* __restrict__ val, const float* __res
     sc->rr = 0.0;
   }
   double pq = 0.0;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < L.count; t += gridDim.x * blockDim.x)
-    mat_rows(L, t, val, p32, [&](int row, double v) {
-      q[row] = v;
-      pq += p[row] * v;
-    });
+  W::rows(L, val, p32, [&](int row, double v) {
+    q[row] = v;
+    pq += p[row] * v;
+  });
   double s = block_sum(pq, sh);
   if (threadIdx.x == 0) atomicAdd(&sc->pq, s);
 }
@@ -516,13 +588,6 @@ inline int red_grid(const gf_ctx* ctx, int64_t work) {
   return std::min(gf_blocks(work, kT), ctx->sm_count * 8);
 }
 
-// grid of the SpMV kernels for layout L (block size L.threads): node blocks run one
-// thread per node (measured faster than a capped grid-stride loop), rows a capped grid
-inline int mat_grid(const gf_ctx* ctx, const MatLayout& L) {
-  if (L.bdim) return gf_blocks(L.count, L.threads);
-  return std::min(gf_blocks(L.count, L.threads), ctx->sm_count * 8);
-}
-
 // The sliced copy of the context's matrix in `dtype` (built or refreshed on demand).
 gf_status solver_matrix(gf_ctx* ctx, int dtype, MatLayout* L, const void** val) {
   gf_status st = gf_sell_prepare(ctx, dtype);
@@ -532,7 +597,7 @@ gf_status solver_matrix(gf_ctx* ctx, int dtype, MatLayout* L, const void** val) 
     L->bdim = ctx->sell_bdim;
     L->nnodes = ctx->nnodes;
     L->perm = ctx->d_sell_perm;
-    L->count = ctx->nnodes;  // a thread per node slot
+    L->split = slice_split(ctx, L->bdim, L->nnodes, ctx->sell_total / 32);
   }
   *val = dtype == GF_F64 ? (const void*)ctx->d_sell_v64 : (const void*)ctx->d_sell_v32;
   return GF_OK;
@@ -551,11 +616,11 @@ gf_status gf_matvec_f32(gf_ctx* ctx, const float* x, const float* scale, float* 
   gf_status st = solver_matrix(ctx, dt, &L, &val);
   if (st != GF_OK) return st;
   if (dt == GF_F64)
-    k_spmv_rowscale<double><<<mat_grid(ctx, L), L.threads, 0, ctx->stream>>>(
-        L, (const double*)val, x, scale, y);
+    GF_ROWS_LAUNCH(ctx, ctx->stream, L, (k_spmv_rowscale<Walk, double>),
+                   (const double*)val, x, scale, y);
   else
-    k_spmv_rowscale<float><<<mat_grid(ctx, L), L.threads, 0, ctx->stream>>>(
-        L, (const float*)val, x, scale, y);
+    GF_ROWS_LAUNCH(ctx, ctx->stream, L, (k_spmv_rowscale<Walk, float>),
+                   (const float*)val, x, scale, y);
   ctx->launches++;
   return GF_OK;
 }
@@ -570,11 +635,11 @@ gf_status gf_spmv_launch(gf_ctx* ctx, int dtype, const void* x, void* y) {
     return gf_fail(ctx, GF_ERR_INVALID_ARG, "x must be aligned to two entries");
   cudaEventRecord(ctx->ev0, ctx->stream);
   if (dtype == GF_F64)
-    k_spmv<double, double, double><<<mat_grid(ctx, L), L.threads, 0, ctx->stream>>>(
-        L, (const double*)val, (const double*)x, (double*)y);
+    GF_ROWS_LAUNCH(ctx, ctx->stream, L, (k_spmv<Walk, double, double, double>),
+                   (const double*)val, (const double*)x, (double*)y);
   else
-    k_spmv<float, float, float><<<mat_grid(ctx, L), L.threads, 0, ctx->stream>>>(
-        L, (const float*)val, (const float*)x, (float*)y);
+    GF_ROWS_LAUNCH(ctx, ctx->stream, L, (k_spmv<Walk, float, float, float>),
+                   (const float*)val, (const float*)x, (float*)y);
   GF_LAUNCH_CHECK(ctx, "k_spmv");
   cudaEventRecord(ctx->ev1, ctx->stream);
   GF_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
@@ -688,7 +753,7 @@ gf_status run_cg(gf_ctx* ctx, MatLayout L, const TK* val, const V* b, CgVecs vv,
   cudaGraphExec_t exec = nullptr;
   GF_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   for (int k = 0; k < check_every; ++k) {
-    k_cg_spmv_dot<TK, V><<<mat_grid(ctx, L), L.threads, 0, s>>>(L, val, p, q, sc);
+    GF_ROWS_LAUNCH(ctx, s, L, (k_cg_spmv_dot<Walk, TK, V>), val, p, q, sc);
     k_cg_update<V><<<red_grid(ctx, n), kT, 0, s>>>(n, x, r, zz, p, q, dinv, sc);
     k_cg_direction<V><<<nb, kT, 0, s>>>(n, zz, p, sc);
   }
@@ -756,8 +821,8 @@ gf_status residual64(gf_ctx* ctx, double* r64, double* rr) {
   const void* val = nullptr;
   gf_status st = solver_matrix(ctx, GF_F64, &L, &val);
   if (st != GF_OK) return st;
-  k_residual64<<<mat_grid(ctx, L), L.threads, 0, s>>>(L, (const double*)val, ctx->d_u, ctx->d_f,
-                                                     r64, ctx->d_red);
+  GF_ROWS_LAUNCH(ctx, s, L, (k_residual64<Walk>),
+                 (const double*)val, ctx->d_u, ctx->d_f, r64, ctx->d_red);
   GF_LAUNCH_CHECK(ctx, "k_residual64");
   double* h = (double*)ctx->h_pinned + 16;
   GF_CUDA(ctx, cudaMemcpyAsync(h, ctx->d_red, sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -904,18 +969,18 @@ gf_status run_mixed(gf_ctx* ctx, const gf_solve_opts* o, int maxit, int check,
     for (int k = 0; k < check; ++k) {
       if (twolevel) {
         if constexpr (sizeof(V) == sizeof(double)) {
-          k_cg_spmv_dot_x32<<<mat_grid(ctx, L32), L32.threads, 0, s>>>(L32, val32, p32, p, q, sc);
+          GF_ROWS_LAUNCH(ctx, s, L32, (k_cg_spmv_dot_x32<Walk>), val32, p32, p, q, sc);
           gf_tl_iterate(ctx, x, r, p, q, dinv, sc, p32);
         } else {
-          k_cg_spmv_dot<float, V><<<mat_grid(ctx, L32), L32.threads, 0, s>>>(L32, val32, p, q, sc);
+          GF_ROWS_LAUNCH(ctx, s, L32, (k_cg_spmv_dot<Walk, float, V>), val32, p, q, sc);
           gf_tl_iterate(ctx, x, r, p, q, dinv, sc);
         }
       } else {
         if (p32)
-          k_cg_spmv_dot_x32<<<mat_grid(ctx, L32), L32.threads, 0, s>>>(
-              L32, val32, p32, (const double*)p, (double*)q, sc);
+          GF_ROWS_LAUNCH(ctx, s, L32, (k_cg_spmv_dot_x32<Walk>),
+                         val32, p32, (const double*)p, (double*)q, sc);
         else
-          k_cg_spmv_dot<float, V><<<mat_grid(ctx, L32), L32.threads, 0, s>>>(L32, val32, p, q, sc);
+          GF_ROWS_LAUNCH(ctx, s, L32, (k_cg_spmv_dot<Walk, float, V>), val32, p, q, sc);
         k_cg_update<V><<<red_grid(ctx, n), kT, 0, s>>>(n, x, r, z, p, q, dinv, sc);
         k_cg_direction<V><<<nb, kT, 0, s>>>(n, z, p, sc, p32);
       }
@@ -1113,19 +1178,19 @@ __global__ void k_fcg_dir(int n, const double* __restrict__ z, double* __restric
   if (i < n) p[i] = z[i] + beta * p[i];
 }
 
-__global__ void __launch_bounds__(kT)
+template <class W>
+__global__ void __launch_bounds__(W::kThreads, 1)
 k_fcg_spmv(MatLayout L, const double* __restrict__ val, const double* __restrict__ p,
            const double* __restrict__ r, double* __restrict__ q, FcgScalars* sc) {
   __shared__ double sh[32];
   if (sc->done) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) sc->rr = 0.0;
   double pq = 0.0, pr = 0.0;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < L.count; t += gridDim.x * blockDim.x)
-    mat_rows(L, t, val, p, [&](int row, double v) {
-      q[row] = v;
-      pq += p[row] * v;
-      pr += p[row] * r[row];
-    });
+  W::rows(L, val, p, [&](int row, double v) {
+    q[row] = v;
+    pq += p[row] * v;
+    pr += p[row] * r[row];
+  });
   double s1 = block_sum(pq, sh);
   if (threadIdx.x == 0) atomicAdd(&sc->pq, s1);
   double s2 = block_sum(pr, sh);
@@ -1236,7 +1301,7 @@ gf_status run_fcg(gf_ctx* ctx, const gf_solve_opts* o, int maxit, int check,
       }
       k_fcg_dots<<<red_grid(ctx, n), kT, 0, s>>>(n, z, r, rold, sc);
       k_fcg_dir<<<nb, kT, 0, s>>>(n, z, p, sc);
-      k_fcg_spmv<<<mat_grid(ctx, L), L.threads, 0, s>>>(L, val, p, r, q, sc);
+      GF_ROWS_LAUNCH(ctx, s, L, (k_fcg_spmv<Walk>), val, p, r, q, sc);
       k_fcg_update<<<red_grid(ctx, n), kT, 0, s>>>(n, x, r, rold, p, q, sc);
       k_fcg_finish<<<1, 1, 0, s>>>(sc);
     }
@@ -1347,8 +1412,7 @@ gf_status gf_pcg_record(gf_ctx* ctx, const double* ustar, int npairs, int every,
   int got = 1;
   while (got < npairs) {
     for (int k = 0; k < every; ++k) {
-      k_cg_spmv_dot<double, double><<<mat_grid(ctx, L), L.threads, 0, s>>>(
-          L, (const double*)vk, p, q, sc);
+      GF_ROWS_LAUNCH(ctx, s, L, (k_cg_spmv_dot<Walk, double, double>), (const double*)vk, p, q, sc);
       if (twolevel) {
         gf_tl_iterate(ctx, x, r, p, q, dinv, sc);
       } else {
@@ -1402,7 +1466,7 @@ gf_status run_twolevel(gf_ctx* ctx, const gf_solve_opts* o, int maxit, int check
   const int64_t l0 = ctx->launches;
   GF_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   for (int k = 0; k < check; ++k) {
-    k_cg_spmv_dot<double, double><<<mat_grid(ctx, L), L.threads, 0, s>>>(L, val, p, q, sc);
+    GF_ROWS_LAUNCH(ctx, s, L, (k_cg_spmv_dot<Walk, double, double>), val, p, q, sc);
     gf_tl_iterate(ctx, x, r, p, q, dinv, sc);
   }
   cudaError_t ce = cudaStreamEndCapture(s, &graph);
@@ -1654,7 +1718,8 @@ __global__ void k_dist_scatter(int m, const int32_t* __restrict__ idx, const dou
 
 // q = K_local p over every local row; p.q over the owned rows only.  Block 0 clears the
 // r.z / r.r slots that the update kernel accumulates into next.
-__global__ void __launch_bounds__(kT)
+template <class W>
+__global__ void __launch_bounds__(W::kThreads, 1)
 k_dist_spmv_dot(MatLayout L, const double* __restrict__ val, const double* __restrict__ p,
                 double* __restrict__ q, int no, DistScalars* sc) {
   __shared__ double sh[32];
@@ -1664,11 +1729,10 @@ k_dist_spmv_dot(MatLayout L, const double* __restrict__ val, const double* __res
     sc->rr = 0.0;
   }
   double pq = 0.0;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < L.count; t += gridDim.x * blockDim.x)
-    mat_rows(L, t, val, p, [&](int row, double v) {
-      q[row] = v;
-      if (row < no) pq += p[row] * v;
-    });
+  W::rows(L, val, p, [&](int row, double v) {
+    q[row] = v;
+    if (row < no) pq += p[row] * v;
+  });
   const double s = block_sum(pq, sh);
   if (threadIdx.x == 0) atomicAdd(&sc->pq, s);
 }
@@ -1822,7 +1886,7 @@ extern "C" GF_API gf_status gf_dist_pcg(gf_ctx* ctx, const gf_solve_opts* o,
         k_dist_scatter<<<gf_blocks(d->n_recv, kT), kT, 0, s>>>(d->n_recv, d->d_recv, d->d_rbuf, p);
         GF_LAUNCH_CHECK(ctx, "k_dist_scatter");
       }
-      k_dist_spmv_dot<<<mat_grid(ctx, L), L.threads, 0, s>>>(L, (const double*)val, p, q, no, sc);
+      GF_ROWS_LAUNCH(ctx, s, L, (k_dist_spmv_dot<Walk>), (const double*)val, p, q, no, sc);
       GF_LAUNCH_CHECK(ctx, "k_dist_spmv_dot");
       if ((st = coll(allreduce(&sc->pq, 1, (void*)s, user), "all-reduce")) != GF_OK) return st;
       k_dist_update<<<red_grid(ctx, no), kT, 0, s>>>(no, x, r, z, p, q, dinv, sc);
@@ -2005,7 +2069,7 @@ extern "C" GF_API gf_status gf_pcg_noalloc(int32_t n, int32_t width, const int32
   SolveScalars hs{};  // pageable host copy: no pinned allocation
   for (;;) {
     for (int k = 0; k < chunk; ++k) {
-      k_cg_spmv_dot<double, double><<<nb, kT, 0, s>>>(L, values, p, q, sc);
+      k_cg_spmv_dot<RowWalk, double, double><<<nb, kT, 0, s>>>(L, values, p, q, sc);
       k_cg_update<double><<<nb, kT, 0, s>>>(n, x, r, z, p, q, dinv, sc);
       k_cg_direction<double><<<nb, kT, 0, s>>>(n, z, p, sc);
     }
@@ -2019,7 +2083,7 @@ extern "C" GF_API gf_status gf_pcg_noalloc(int32_t n, int32_t width, const int32
   double rr = 0.0;
   e = cudaMemsetAsync(acc, 0, sizeof(double), s);
   if (e != cudaSuccess) return fail(e);
-  k_residual64<<<nb, kT, 0, s>>>(L, values, x, b, r, acc);
+  k_residual64<RowWalk><<<nb, kT, 0, s>>>(L, values, x, b, r, acc);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail(e);
   e = cudaMemcpyAsync(&rr, acc, sizeof(double), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
