@@ -17,7 +17,9 @@
 //
 // One application: restriction (block per aggregate over its node list), the coarse
 // product from the packed upper triangle of the symmetric inverse (64 x 64 tiles, read
-// once at half the size), prolongation fused with the Jacobi term and the r.z dot.  Everything is launched on the context stream without synchronisation.
+// once at half the size), prolongation fused with the Jacobi term and the r.z dot.  In the
+// PCG the restriction comes with the update of x and r, the prolongation with the new
+// direction.  Everything is launched on the context stream without synchronisation.
 #include <cub/cub.cuh>
 #include <algorithm>
 #include <cmath>
@@ -52,8 +54,8 @@ struct Coarse {
   int ntiles = 0;                 // nt (nt + 1) / 2 tiles (I <= J) of the symmetric inverse
   int2* tile_ij = nullptr;        // [ntiles] (I, J)
   double* ainv = nullptr;         // [ntiles][64][64], zero beyond nc
-  unsigned* counter = nullptr;    // blocks done in the current coarse product
-  double* rc = nullptr;          // [nc]
+  int parts = 1;                  // blocks per aggregate of the fused update
+  double* rc = nullptr;          // [parts][64 nt], partial sums of P^T r
   double* zc = nullptr;          // [64 nt]
 };
 
@@ -742,11 +744,11 @@ __global__ void k_pack_tiles(int nc, const int2* __restrict__ ij, const double* 
 
 // rc = P^T r (and zc = 0 for the coarse product): block per aggregate over its node list
 constexpr int kRT = 256;
-template <int DIM, typename V>
+template <int DIM>
 __global__ void __launch_bounds__(kRT)
 k_restrict(const int32_t* __restrict__ off, const int32_t* __restrict__ nodes,
            const double* __restrict__ x, const double* __restrict__ cen, double sinv,
-           const uint8_t* __restrict__ fixed, const V* __restrict__ r,
+           const uint8_t* __restrict__ fixed, const double* __restrict__ r,
            double* __restrict__ rc, double* __restrict__ zc, const int* __restrict__ done) {
   constexpr int NM = DIM == 2 ? 3 : 6;
   __shared__ double ws[kRT / 32][NM];
@@ -766,7 +768,7 @@ k_restrict(const int32_t* __restrict__ off, const int32_t* __restrict__ nodes,
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
       if (fixed[a * DIM + c]) continue;
-      const double rv = (double)r[a * DIM + c];
+      const double rv = r[a * DIM + c];
       double pr[NM];
       p_row<DIM>(c, d, pr);
 #pragma unroll
@@ -789,48 +791,70 @@ k_restrict(const int32_t* __restrict__ off, const int32_t* __restrict__ nodes,
   }
 }
 
-// zc += Ainv rc from the packed upper-triangle tiles: block per tile (I, J) adds A_IJ rc_J
-// to zc_I and, off the diagonal, A_IJ^T rc_I to zc_J (double atomics; zc is zeroed by the
-// restriction), so the symmetric inverse is read once at half its size.  Warp w reads
-// rows 8w .. 8w+7 of the tile as 16-byte pairs, one contiguous 512-byte row per load
-// (lane l: columns 2l, 2l+1).  Row sums: a butterfly that halves the 8 partial sums per
-// step (9 shuffles); column sums: per thread over its 8 rows, then over the warps in
-// shared memory.  With sc: the last block to finish (counter, after a fence) adds
-// rc.zc to sc->rzn and resets the counter.
-__global__ void __launch_bounds__(256)
-k_coarse_symv(int nc, const int2* __restrict__ ij, const double* __restrict__ T,
-              const double* __restrict__ rc, double* __restrict__ zc, unsigned* counter,
-              SolveScalars* sc, const int* __restrict__ done) {
-  __shared__ double xI[kTS], xJ[kTS], colp[8][kTS], red[8];
-  __shared__ bool last;
-  if (done && *done) return;
-  const int2 t = ij[blockIdx.x];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  if (tid < kTS) xI[tid] = rc[t.x * kTS + tid];
-  else if (tid < 2 * kTS) xJ[tid - kTS] = rc[t.y * kTS + tid - kTS];
-  __syncthreads();
-  const double2* base =
-      reinterpret_cast<const double2*>(T + (int64_t)blockIdx.x * kTS * kTS + w * 8 * kTS);
-  double2 a[8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c) a[c] = __ldcs(base + c * 32 + lane);
-  const double x0 = xJ[2 * lane], x1 = xJ[2 * lane + 1];
-  double rs[8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c) rs[c] = a[c].x * x0 + a[c].y * x1;
+// Sums eight values per lane over a warp by halving butterflies (9 shuffles); lane l then holds
+// the sum of value l / 4.
+__device__ inline double warp_sum8(const double (&e)[8]) {
+  const int lane = threadIdx.x & 31;
   const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
   double v4[4], v2[2];
 #pragma unroll
   for (int k = 0; k < 4; ++k)
-    v4[k] = (u16 ? rs[4 + k] : rs[k]) + __shfl_xor_sync(0xffffffffu, u16 ? rs[k] : rs[4 + k], 16);
+    v4[k] = (u16 ? e[4 + k] : e[k]) + __shfl_xor_sync(0xffffffffu, u16 ? e[k] : e[4 + k], 16);
 #pragma unroll
   for (int k = 0; k < 2; ++k)
     v2[k] = (u8 ? v4[2 + k] : v4[k]) + __shfl_xor_sync(0xffffffffu, u8 ? v4[k] : v4[2 + k], 8);
   double v = (u4 ? v2[1] : v2[0]) + __shfl_xor_sync(0xffffffffu, u4 ? v2[0] : v2[1], 4);
   v += __shfl_xor_sync(0xffffffffu, v, 2);
   v += __shfl_xor_sync(0xffffffffu, v, 1);
-  if ((lane & 3) == 0) atomicAdd(&zc[t.x * kTS + w * 8 + (lane >> 2)], v);
-  if (t.x != t.y) {
+  return v;
+}
+
+// zc += Ainv rc from the packed upper-triangle tiles: block per tile (I, J) adds A_IJ rc_J
+// to zc_I and, off the diagonal, A_IJ^T rc_I to zc_J (double atomics; zc is zeroed by the
+// restriction), so the symmetric inverse is read once at half its size.  rc is the sum of
+// `parts` partial vectors of length ld.  Warp w reads rows 8w .. 8w+7 of the tile as 16-byte
+// pairs, one contiguous 512-byte row per load (lane l: columns 2l, 2l+1), all in flight before
+// rc is looked at, and kept in L2 from one iteration to the next.  Column sums: per thread over
+// its 8 rows, then over the warps in shared memory.  With sc: the block adds its part of
+// rc.zc = rc^T Ainv rc to sc->rzn (an off-diagonal tile counts twice); a sum over the finished
+// zc by the last block to end took the kernel's tail (fence, counter, one block reading zc).
+__global__ void __launch_bounds__(256)
+k_coarse_symv(const int2* __restrict__ ij, const double* __restrict__ T,
+              const double* __restrict__ rc, int parts, int ld, double* __restrict__ zc,
+              SolveScalars* sc, const int* __restrict__ done) {
+  __shared__ double xI[kTS], xJ[kTS], colp[8][kTS], red[8];
+  if (done && *done) return;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const double2* base =
+      reinterpret_cast<const double2*>(T + (int64_t)blockIdx.x * kTS * kTS + w * 8 * kTS);
+  double2 a[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) a[c] = __ldg(base + c * 32 + lane);
+  const int2 t = ij[blockIdx.x];
+  if (tid < 2 * kTS) {
+    const double* src = rc + (tid < kTS ? t.x * kTS + tid : t.y * kTS + tid - kTS);
+    double v = 0.0;
+    for (int k = 0; k < parts; ++k) v += src[(int64_t)k * ld];
+    (tid < kTS ? xI[tid] : xJ[tid - kTS]) = v;
+  }
+  __syncthreads();
+  const double x0 = xJ[2 * lane], x1 = xJ[2 * lane + 1];
+  double rs[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) rs[c] = a[c].x * x0 + a[c].y * x1;
+  const double v = warp_sum8(rs);
+  const bool off = t.x != t.y;
+  double part = 0.0;
+  if ((lane & 3) == 0) {
+    const int row = w * 8 + (lane >> 2);
+    atomicAdd(&zc[t.x * kTS + row], v);
+    part = v * xI[row];
+  }
+  if (sc) {
+    for (int o = 16; o > 2; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
+    if (lane == 0) red[w] = part;
+  }
+  if (off) {
     double cx = 0.0, cy = 0.0;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
@@ -840,31 +864,19 @@ k_coarse_symv(int nc, const int2* __restrict__ ij, const double* __restrict__ T,
     }
     colp[w][2 * lane] = cx;
     colp[w][2 * lane + 1] = cy;
-    __syncthreads();
-    if (tid < kTS) {
-      double u = 0.0;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) u += colp[q][tid];
-      atomicAdd(&zc[t.y * kTS + tid], u);
-    }
   }
-  if (!sc) return;
-  __threadfence();
   __syncthreads();
-  if (tid == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double part = 0.0;
-  for (int j = tid; j < nc; j += blockDim.x) part += rc[j] * __ldcg(zc + j);
-  for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
-  if (lane == 0) red[w] = part;
-  __syncthreads();
-  if (tid == 0) {
+  if (off && tid < kTS) {
     double u = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) u += colp[q][tid];
+    atomicAdd(&zc[t.y * kTS + tid], u);
+  }
+  if (sc && tid == kTS) {
+    double u = 0.0;
+#pragma unroll
     for (int q = 0; q < 8; ++q) u += red[q];
-    atomicAdd(&sc->rzn, u);
-    *counter = 0u;
+    atomicAdd(&sc->rzn, off ? 2.0 * u : u);
   }
 }
 
@@ -919,57 +931,107 @@ k_prolong(int n, const int32_t* __restrict__ agg, const double* __restrict__ x,
 // The direction kernel forms z = D^-1 r + P zc on the fly, using
 //   r.z = r.D^-1 r + (P^T r).zc = r.D^-1 r + rc.zc,
 // so z is never stored: r.D^-1 r comes with the x/r update, rc.zc with the coarse
-// product.  (Folding the restriction into the update as well, with warp-aggregated
-// atomics per aggregate, measured slower than the block-per-aggregate kernel: the
-// shuffles cost more than the second read of r.)
+// product.
 
 // INIT: x = 0, r = scale * b.  Else: alpha = rz / p.q, x += alpha p, r -= alpha q.
-// Accumulates rr = r.r and rzn += r.D^-1 r (in FP64 whatever the vector type V).
-template <bool INIT, typename V>
-__global__ void __launch_bounds__(kCT)
-k_tl_update(int n, const double* __restrict__ b, const V* __restrict__ q, double scale,
-            V* __restrict__ x, V* __restrict__ r, const V* __restrict__ p,
-            const V* __restrict__ dinv, SolveScalars* sc) {
-  __shared__ double sh[32];
+// Accumulates rr = r.r and rzn += r.D^-1 r (in FP64 whatever the vector type V), and restricts
+// r: every node is in one aggregate, so a block walks its share (blockIdx.y of gridDim.y) of
+// aggregate blockIdx.x's node list, updates those nodes' entries and leaves the share's sums of
+// P^T r in rc[blockIdx.y]; the block of share 0 zeroes the aggregate's part of zc for the
+// coarse product.  Bound by latency at the sizes where it matters (182k dofs: 1.4 MB per
+// vector, in L2), hence one thread per node with all of its entries' loads in flight, enough
+// shares per aggregate for one or two nodes per thread, and one warp reduction for the eight
+// sums.  As two kernels, x/r by rows and the restriction by a block per aggregate, it was a
+// launch and a second pass over r more.  An iteration with this, the coarse product's own r.z
+// and the direction per node: Brick20 24^3 FP64 64.2 -> 58.2 us, 14^3 26.7 -> 22.6, Q8 128
+// 23.3 -> 18.5; from 600k dofs on no difference.
+constexpr int kUT = 128;
+template <int DIM, bool INIT, typename V>
+__global__ void __launch_bounds__(kUT, 1)
+k_tl_update(const int32_t* __restrict__ off, const int32_t* __restrict__ nodes,
+            const double* __restrict__ xc, const double* __restrict__ cen, double sinv,
+            const uint8_t* __restrict__ fixed, const double* __restrict__ b,
+            const V* __restrict__ q, double scale, V* __restrict__ x, V* __restrict__ r,
+            const V* __restrict__ p, const V* __restrict__ dinv, double* __restrict__ rc, int ld,
+            double* __restrict__ zc, SolveScalars* sc) {
+  constexpr int NM = DIM == 2 ? 3 : 6;
+  static_assert(NM + 2 <= 8, "sums per warp reduction");
+  __shared__ double ws[kUT / 32][8];
   double alpha = 0.0;
   if (!INIT) {
     if (sc->done) return;
     const double pq = sc->pq;
     if (!(pq > 0.0) || !isfinite(pq)) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) sc->done = 2;
+      if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) sc->done = 2;
       return;
     }
     alpha = sc->rz / pq;
   }
-  double rr = 0.0, rdr = 0.0;
-  for (int i = blockIdx.x * kCT + threadIdx.x; i < n; i += gridDim.x * kCT) {
-    V ri;
-    if (INIT) {
-      ri = (V)(b[i] * scale);
-      x[i] = V(0);
-    } else {
-      x[i] += (V)alpha * p[i];
-      ri = r[i] - (V)alpha * q[i];
+  const int A = blockIdx.x;
+  double cA[DIM];
+#pragma unroll
+  for (int c = 0; c < DIM; ++c) cA[c] = cen[(int64_t)A * DIM + c];
+  double acc[8];  // the modes, r.r, r.D^-1 r
+#pragma unroll
+  for (int m = 0; m < 8; ++m) acc[m] = 0.0;
+  const int end = off[A + 1];
+  for (int t = off[A] + blockIdx.y * kUT + threadIdx.x; t < end; t += gridDim.y * kUT) {
+    const int a = nodes[t];
+    const int64_t i = (int64_t)a * DIM;
+    double d[DIM], f[DIM];
+    V ri[DIM];
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      d[c] = (xc[i + c] - cA[c]) * sinv;
+      f[c] = (double)dinv[i + c];
+      if (INIT) {
+        ri[c] = (V)(b[i + c] * scale);
+        x[i + c] = V(0);
+      } else {
+        x[i + c] += (V)alpha * p[i + c];
+        ri[c] = r[i + c] - (V)alpha * q[i + c];
+      }
+      r[i + c] = ri[c];
     }
-    r[i] = ri;
-    const double rd = (double)ri;
-    rr += rd * rd;
-    rdr += rd * rd * (double)dinv[i];
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      const double rd = (double)ri[c];
+      acc[NM] += rd * rd;
+      acc[NM + 1] += rd * rd * f[c];
+      if (fixed[i + c]) continue;
+      double pr[NM];
+      p_row<DIM>(c, d, pr);
+#pragma unroll
+      for (int m = 0; m < NM; ++m) acc[m] += pr[m] * rd;
+    }
   }
-  const double s1 = cg_block_sum(rr, sh);
-  if (threadIdx.x == 0) atomicAdd(&sc->rr, s1);
-  const double s2 = cg_block_sum(rdr, sh);
-  if (threadIdx.x == 0) atomicAdd(&sc->rzn, s2);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const double v = warp_sum8(acc);
+  if ((l & 3) == 0) ws[w][l >> 2] = v;
+  __syncthreads();
+  const int m = threadIdx.x;
+  if (m < NM + 2) {
+    double u = 0.0;
+#pragma unroll
+    for (int k = 0; k < kUT / 32; ++k) u += ws[k][m];
+    if (m < NM) {
+      rc[(int64_t)blockIdx.y * ld + A * NM + m] = u;
+      if (blockIdx.y == 0) zc[A * NM + m] = 0.0;
+    } else {
+      atomicAdd(m == NM ? &sc->rr : &sc->rzn, u);
+    }
+  }
 }
 
 // z = D^-1 r + P zc on the fly.  MODE kTlFirst: p = z; kTlKeep: p = pscale p (a
 // reliable update that keeps the direction); kTlStep: p = z + beta p with
 // beta = rzn / rz, then the iteration count and the convergence test.  p32 (or null)
-// receives an FP32 copy of p for SpMVs on the FP32 matrix.
+// receives an FP32 copy of p for SpMVs on the FP32 matrix.  A thread per node: its aggregate,
+// offset and coarse values are read once for all of its rows.
 constexpr int kTlFirst = 0, kTlKeep = 1, kTlStep = 2;
 template <int DIM, int MODE, typename V>
-__global__ void __launch_bounds__(kCT)
-k_tl_direction(int n, const V* __restrict__ r, const V* __restrict__ dinv,
+__global__ void __launch_bounds__(kCT, 1)
+k_tl_direction(int nnodes, const V* __restrict__ r, const V* __restrict__ dinv,
                const uint8_t* __restrict__ fixed, const int32_t* __restrict__ agg,
                const double* __restrict__ xc, const double* __restrict__ cen, double sinv,
                const double* __restrict__ zc, V* __restrict__ p, float* __restrict__ p32,
@@ -977,6 +1039,7 @@ k_tl_direction(int n, const V* __restrict__ r, const V* __restrict__ dinv,
   constexpr int NM = DIM == 2 ? 3 : 6;
   if (sc->done) return;
   if (MODE == kTlKeep) {
+    const int64_t n = (int64_t)nnodes * DIM;
     for (int64_t t = (int64_t)blockIdx.x * kCT + threadIdx.x; t < n; t += (int64_t)gridDim.x * kCT) {
       const V pn = (V)((double)p[t] * pscale);
       p[t] = pn;
@@ -985,25 +1048,27 @@ k_tl_direction(int n, const V* __restrict__ r, const V* __restrict__ dinv,
     return;
   }
   const double beta = MODE == kTlFirst ? 0.0 : sc->rzn / sc->rz;
-  const int64_t stride = (int64_t)gridDim.x * kCT;
-  for (int64_t t = (int64_t)blockIdx.x * kCT + threadIdx.x; t < n; t += stride) {
-    const int i = (int)t;
-    double zi = (double)dinv[i] * (double)r[i];
-    if (!fixed[i]) {
-      const int a = i / DIM, c = i - a * DIM;
-      const int A = agg[a];
-      double d[DIM];
+  for (int a = blockIdx.x * kCT + threadIdx.x; a < nnodes; a += gridDim.x * kCT) {
+    const int64_t i = (int64_t)a * DIM;
+    const int A = agg[a];
+    double d[DIM], zA[NM];
 #pragma unroll
-      for (int k = 0; k < DIM; ++k)
-        d[k] = (xc[(int64_t)a * DIM + k] - cen[(int64_t)A * DIM + k]) * sinv;
-      double pr[NM];
-      p_row<DIM>(c, d, pr);
+    for (int k = 0; k < DIM; ++k) d[k] = (xc[i + k] - cen[(int64_t)A * DIM + k]) * sinv;
 #pragma unroll
-      for (int m = 0; m < NM; ++m) zi += pr[m] * zc[A * NM + m];
+    for (int m = 0; m < NM; ++m) zA[m] = zc[A * NM + m];
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      double zi = (double)dinv[i + c] * (double)r[i + c];
+      if (!fixed[i + c]) {
+        double pr[NM];
+        p_row<DIM>(c, d, pr);
+#pragma unroll
+        for (int m = 0; m < NM; ++m) zi += pr[m] * zA[m];
+      }
+      const V pn = (V)(MODE == kTlFirst ? zi : zi + beta * (double)p[i + c]);
+      p[i + c] = pn;
+      if (p32) p32[i + c] = (float)pn;
     }
-    const V pn = (V)(MODE == kTlFirst ? zi : zi + beta * (double)p[i]);
-    p[i] = pn;
-    if (p32) p32[i] = (float)pn;
   }
   if (MODE == kTlStep && blockIdx.x == 0 && threadIdx.x == 0) {
     sc->pq = 0.0;
@@ -1020,7 +1085,6 @@ void coarse_release(gf_ctx* ctx, Coarse* c) {
   gf_pfree(ctx, c->cen);
   gf_pfree(ctx, c->ainv);
   gf_pfree(ctx, c->tile_ij);
-  gf_pfree(ctx, c->counter);
   gf_pfree(ctx, c->rc);
   gf_pfree(ctx, c->zc);
 }
@@ -1104,6 +1168,7 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
   const int ld = nt * kTS;  // length of rc, zc
   C->nt = nt;
   C->ntiles = ntiles;
+  C->parts = std::max(1, std::min(gf_blocks(nnodes, kUT * na), 16 * ctx->sm_count / na));
   C->dim = dim; C->nm = nm; C->na = na; C->nc = nc; C->s = side;
   for (int c = 0; c < 3; ++c) { C->lo[c] = g.lo[c]; C->nb[c] = g.nb[c]; }
   double* d_Ac = nullptr;
@@ -1122,8 +1187,7 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
       (st = gf_palloc(ctx, &C->cen, (size_t)na * dim)) != GF_OK ||
       (st = gf_palloc(ctx, &C->ainv, (size_t)ntiles * kTS * kTS)) != GF_OK ||
       (st = gf_palloc(ctx, &C->tile_ij, (size_t)ntiles)) != GF_OK ||
-      (st = gf_palloc(ctx, &C->counter, 1)) != GF_OK ||
-      (st = gf_palloc(ctx, &C->rc, (size_t)ld)) != GF_OK ||
+      (st = gf_palloc(ctx, &C->rc, (size_t)ld * C->parts)) != GF_OK ||
       (st = gf_palloc(ctx, &C->zc, (size_t)ld)) != GF_OK ||
       (st = gf_palloc(ctx, &d_Ac, (size_t)nc * nc)) != GF_OK ||
       (st = gf_palloc(ctx, &d_pi, (size_t)kGJ * kGJ)) != GF_OK ||
@@ -1226,9 +1290,8 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
   GF_CUDA(ctx, cudaMemcpyAsync(C->tile_ij, hij.data(), sizeof(int2) * ntiles,
                                cudaMemcpyHostToDevice, s));
   k_pack_tiles<<<ntiles, 256, 0, s>>>(nc, C->tile_ij, d_Ac, C->ainv);
-  cudaMemsetAsync(C->rc, 0, sizeof(double) * ld, s);  // the tails beyond nc stay zero
+  cudaMemsetAsync(C->rc, 0, sizeof(double) * ld * C->parts, s);  // the tails beyond nc stay zero
   cudaMemsetAsync(C->zc, 0, sizeof(double) * ld, s);
-  cudaMemsetAsync(C->counter, 0, sizeof(unsigned), s);
   ctx->launches++;
   cudaError_t e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = cudaGetLastError();
@@ -1276,17 +1339,17 @@ static void coarse_apply_impl(gf_ctx* ctx, const double* r, const double* dinv, 
   const double sinv = 1.0 / c->s;
   const int pb = std::min(gf_blocks(ctx->n, kCT), ctx->sm_count * 8);
   if (c->dim == 2) {
-    k_restrict<2, double><<<c->na, kRT, 0, s>>>(c->agg_off, c->agg_nodes, ctx->d_coords64, c->cen, sinv,
+    k_restrict<2><<<c->na, kRT, 0, s>>>(c->agg_off, c->agg_nodes, ctx->d_coords64, c->cen, sinv,
                                         ctx->d_fixed, r, c->rc, c->zc, done);
-    k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->nc, c->tile_ij, c->ainv, c->rc, c->zc, nullptr,
-                                            nullptr, done);
+    k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->tile_ij, c->ainv, c->rc, 1, 0, c->zc, nullptr,
+                                            done);
     k_prolong<2><<<pb, kCT, 0, s>>>(ctx->n, c->node_agg, ctx->d_coords64, c->cen, sinv,
                                     ctx->d_fixed, dinv, r, c->zc, z, rz_acc, done, add);
   } else {
-    k_restrict<3, double><<<c->na, kRT, 0, s>>>(c->agg_off, c->agg_nodes, ctx->d_coords64, c->cen, sinv,
+    k_restrict<3><<<c->na, kRT, 0, s>>>(c->agg_off, c->agg_nodes, ctx->d_coords64, c->cen, sinv,
                                         ctx->d_fixed, r, c->rc, c->zc, done);
-    k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->nc, c->tile_ij, c->ainv, c->rc, c->zc, nullptr,
-                                            nullptr, done);
+    k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->tile_ij, c->ainv, c->rc, 1, 0, c->zc, nullptr,
+                                            done);
     k_prolong<3><<<pb, kCT, 0, s>>>(ctx->n, c->node_agg, ctx->d_coords64, c->cen, sinv,
                                     ctx->d_fixed, dinv, r, c->zc, z, rz_acc, done, add);
   }
@@ -1308,31 +1371,28 @@ static void tl_launch(gf_ctx* ctx, int mode, const double* b, const V* q, double
                       float* p32) {
   Coarse* c = static_cast<Coarse*>(ctx->coarse);
   cudaStream_t s = ctx->stream;
-  const int n = ctx->n;
+  const int nn = ctx->nnodes, ld = c->nt * kTS;
   const double sinv = 1.0 / c->s;
-  const int grid = std::min(gf_blocks(n, kCT), ctx->sm_count * 8);
-  if (mode == kTlStep)
-    k_tl_update<false, V><<<grid, kCT, 0, s>>>(n, nullptr, q, 1.0, x, r, p, dinv, sc);
-  else
-    k_tl_update<true, V><<<grid, kCT, 0, s>>>(n, b, nullptr, scale, x, r, nullptr, dinv, sc);
-  k_restrict<DIM, V><<<c->na, kRT, 0, s>>>(c->agg_off, c->agg_nodes, ctx->d_coords64, c->cen,
-                                           sinv, ctx->d_fixed, r, c->rc, c->zc, &sc->done);
-  k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->nc, c->tile_ij, c->ainv, c->rc, c->zc, c->counter,
-                                          sc, &sc->done);
+  const int grid = std::min(gf_blocks(nn, kCT), ctx->sm_count * 8);
   const uint8_t* fx = ctx->d_fixed;
-  if (mode == kTlFirst)
-    k_tl_direction<DIM, kTlFirst, V><<<grid, kCT, 0, s>>>(n, r, dinv, fx, c->node_agg,
-                                                          ctx->d_coords64, c->cen, sinv, c->zc,
-                                                          p, p32, 1.0, sc);
-  else if (mode == kTlKeep)
-    k_tl_direction<DIM, kTlKeep, V><<<grid, kCT, 0, s>>>(n, r, dinv, fx, c->node_agg,
-                                                         ctx->d_coords64, c->cen, sinv, c->zc,
-                                                         p, p32, pscale, sc);
+  const double* xc = ctx->d_coords64;
+  const dim3 gu(c->na, c->parts);
+  if (mode == kTlStep)
+    k_tl_update<DIM, false, V><<<gu, kUT, 0, s>>>(c->agg_off, c->agg_nodes, xc, c->cen, sinv, fx,
+                                                  nullptr, q, 1.0, x, r, p, dinv, c->rc, ld,
+                                                  c->zc, sc);
   else
-    k_tl_direction<DIM, kTlStep, V><<<grid, kCT, 0, s>>>(n, r, dinv, fx, c->node_agg,
-                                                         ctx->d_coords64, c->cen, sinv, c->zc,
-                                                         p, p32, 1.0, sc);
-  ctx->launches += 4;
+    k_tl_update<DIM, true, V><<<gu, kUT, 0, s>>>(c->agg_off, c->agg_nodes, xc, c->cen, sinv, fx, b,
+                                                 nullptr, scale, x, r, nullptr, dinv, c->rc, ld,
+                                                 c->zc, sc);
+  k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->tile_ij, c->ainv, c->rc, c->parts, ld, c->zc, sc,
+                                          &sc->done);
+  auto* direction = mode == kTlFirst  ? k_tl_direction<DIM, kTlFirst, V>
+                    : mode == kTlKeep ? k_tl_direction<DIM, kTlKeep, V>
+                                      : k_tl_direction<DIM, kTlStep, V>;
+  direction<<<grid, kCT, 0, s>>>(nn, r, dinv, fx, c->node_agg, xc, c->cen, sinv, c->zc, p, p32,
+                                 pscale, sc);
+  ctx->launches += 3;
 }
 
 template <typename V>
