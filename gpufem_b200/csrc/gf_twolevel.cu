@@ -11,9 +11,9 @@
 // (offsets d = (x - c_A) / s, s = the box side); rows of constrained dofs are zero.
 // M is symmetric positive definite, so plain PCG applies.  The coarse matrix
 // Ac = P^T K P is assembled on the device from the ELL node blocks, regularised by
-// 1e-10 * max diag (modes that the constraints pin down), and inverted in place by a
-// blocked Gauss-Jordan sweep (SPD: no pivoting); the inverse is symmetrised and kept in
-// FP64 for the per-iteration product.
+// 1e-10 * max diag (modes that the constraints pin down), and inverted in place by blocked
+// symmetric sweeps (SPD: no pivoting); the inverse is kept in FP64 for the per-iteration
+// product.
 //
 // One application: restriction (block per aggregate over its node list), the coarse
 // product from the packed upper triangle of the symmetric inverse (64 x 64 tiles, read
@@ -33,11 +33,10 @@ constexpr int kCT = 256;
 constexpr int kMaxCoarse = 4096;
 constexpr int kDefaultCoarse = 3072;
 
-// Default coarse size: n / 128 within [192, 3072].  The set-up (the Gauss-Jordan sweep is
-// O(nc^3)) costs ~10 ms at nc = 3072 whatever the mesh; measured on B200 with set-up
-// and solve to 1e-8 together, n / 128 is the fastest of nc = 3072, n/16, n/32, n/64 and
-// n/128 on Brick8 cubes of 15k-353k dofs and Q8 128^2 (e.g. 207k dofs: 7.5 ms against
-// 14.3 ms at nc = 3072); from 393k dofs on the default is 3072.
+// Default coarse size: n / 128 within [192, 3072].  The set-up (the inversion is O(nc^3))
+// costs 1.3 ms at nc = 1296 and 3 ms at nc = 3072.  Chosen with set-up and solve to 1e-8 together
+// when the inversion took twice as long: n / 128 was the fastest of nc = 3072, n/16, n/32, n/64
+// and n/128 on Brick8 cubes of 15k-353k dofs and Q8 128^2; from 393k dofs on the default is 3072.
 inline int default_coarse(int n) { return std::min(kDefaultCoarse, std::max(192, n / 128)); }
 
 struct Coarse {
@@ -517,116 +516,24 @@ __global__ void k_regularise(int nc, const double* __restrict__ dmax, double eps
   d = d > 0.0 ? d + eps * (*dmax) : 1.0;
 }
 
-// Blocked Gauss-Jordan sweep (in place, SPD: no pivoting).  For the pivot block P of
-// kGJ rows/columns at kb and the rest R:
-//   A_PP <- A_PP^-1,  A_PR <- A_PP^-1 A_PR,  A_RP <- -A_RP A_PP^-1,
-//   A_RR <- A_RR - A_RP A_PP^-1 A_PR
-// After a sweep over every block A holds its inverse.  Three kernels per block:
-// the pivot block's inverse (one CTA), the two panels, and the rank-kGJ update; the
-// panels and the update are 64 x 64 output tiles of 64-deep products (4 x 4 outputs per
-// thread from shared-memory operands), so every pass over A does 64 FMAs per entry.
-constexpr int kGJ = 64;
-constexpr int kGT = 64;                 // output tile side
-constexpr int kGJRows = 16;             // pivot CTA: kGJ x kGJRows threads, 4 rows each
-constexpr size_t kGJSmem = sizeof(double) * ((size_t)kGT * (kGJ + 1) + (size_t)kGJ * kGT);
-
-// Pi = A_PP^-1 by scalar sweeps in shared memory (bs <= kGJ)
-__global__ void __launch_bounds__(kGJ * kGJRows)
-k_gj_pivot(int nc, int kb, int bs, const double* __restrict__ A, double* __restrict__ Pi) {
-  __shared__ double M[kGJ][kGJ + 1];
-  __shared__ double row[kGJ], col[kGJ], piv;
-  const int j = threadIdx.x, i0 = threadIdx.y;
-  for (int i = i0; i < kGJ; i += kGJRows)
-    M[i][j] = (i < bs && j < bs) ? A[(int64_t)(kb + i) * nc + kb + j] : 0.0;
-  __syncthreads();
-  for (int k = 0; k < bs; ++k) {
-    if (i0 == 0) row[j] = M[k][j];
-    if (i0 == 1) col[j] = M[j][k];
-    if (i0 == 2 && j == 0) piv = 1.0 / M[k][k];   // one division per step
-    __syncthreads();
-    const double p = piv;
-    if (j < bs)
-      for (int i = i0; i < bs; i += kGJRows) {
-        double v;
-        if (i == k && j == k) v = p;
-        else if (i == k) v = row[j] * p;
-        else if (j == k) v = -col[i] * p;
-        else v = M[i][j] - col[i] * row[j] * p;
-        M[i][j] = v;
-      }
-    __syncthreads();
-  }
-  for (int i = i0; i < kGJ; i += kGJRows) Pi[i * kGJ + j] = M[i][j];
-}
-
-// acc[a][b] = sum_u X[ty + 16a][u] Y[u][tx + 16b] over u < kGJ (X rows padded to kGJ + 1)
-__device__ __forceinline__ void gj_tile_product(const double (*X)[kGJ + 1],
-                                                const double (*Y)[kGT], double (&acc)[4][4]) {
-  const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-#pragma unroll 8
-  for (int u = 0; u < kGJ; ++u) {
-    double cv[4], rv[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) cv[a] = X[ty + 16 * a][u];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) rv[b] = Y[u][tx + 16 * b];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] += cv[a] * rv[b];
-  }
-}
-
-// blockIdx.y = 0: row panel Rw[r][j] = sum_u Pi[r][u] A[kb+u][j] for the 64 columns j0..
-// blockIdx.y = 1: column panel Cold[i][t] = A[i][kb+t], Cn[i][t] = -sum_u A[i][kb+u] Pi[u][t]
-__global__ void __launch_bounds__(256)
-k_gj_panels(int nc, int kb, int bs, const double* __restrict__ A, const double* __restrict__ Pi,
-            double* __restrict__ Rw, double* __restrict__ Cold, double* __restrict__ Cn) {
-  extern __shared__ __align__(16) double gsm[];
-  double (*X)[kGJ + 1] = reinterpret_cast<double (*)[kGJ + 1]>(gsm);
-  double (*Y)[kGT] = reinterpret_cast<double (*)[kGT]>(gsm + kGT * (kGJ + 1));
-  const int t0 = blockIdx.x * kGT;
-  const bool rowp = blockIdx.y == 0;
-  for (int e = threadIdx.x; e < kGT * kGJ; e += 256) {
-    const int r = e / kGJ, u = e % kGJ;      // X[r][u]
-    const int u2 = e / kGT, c2 = e % kGT;    // Y[u2][c2]
-    if (rowp) {
-      X[r][u] = Pi[r * kGJ + u];
-      Y[u2][c2] = (u2 < bs && t0 + c2 < nc) ? A[(int64_t)(kb + u2) * nc + t0 + c2] : 0.0;
-    } else {
-      X[r][u] = (u < bs && t0 + r < nc) ? A[(int64_t)(t0 + r) * nc + kb + u] : 0.0;
-      Y[u2][c2] = Pi[u2 * kGJ + c2];
-    }
-  }
-  __syncthreads();
-  double acc[4][4];
-  gj_tile_product(X, Y, acc);
-  const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int r = ty + 16 * a, c = tx + 16 * b;
-      if (rowp) {
-        if (r < bs && t0 + c < nc) Rw[(int64_t)r * nc + t0 + c] = acc[a][b];
-      } else if (t0 + r < nc && c < bs) {
-        Cold[(int64_t)(t0 + r) * kGJ + c] = X[r][c];
-        Cn[(int64_t)(t0 + r) * kGJ + c] = -acc[a][b];
-      }
-    }
-}
-
-// Every entry (i, j): a 64 x 64 tile per CTA of four warps, each warp a 32 x 32 quarter
-// as 4 x 4 fragments of the FP64 tensor-core product mma.m8n8k4 (per lane: one A value
-// A[g][t], one B value B[t][g], two accumulators D[g][2t], D[g][2t + 1] with g = lane / 4,
-// t = lane % 4).  The Cold rows and Rw columns of the tile sit in shared memory with rows
-// of kGJ + 4 doubles (the fragment loads of a warp fall on distinct bank pairs).
-constexpr int kGU = kGJ + 4;   // shared row length (doubles) of the update's operand tiles
-constexpr size_t kGJUpdateSmem = sizeof(double) * 2 * (size_t)kGT * kGU;
+// Inversion by blocked symmetric sweeps (SPD: no pivoting), in place on the upper-triangle
+// tiles (I <= J) of 64 x 64 that the coarse product reads later, padded with the identity to
+// whole tiles.  Sweeping block K:
+//   D = A_KK^-1,  A_KK <- -D,  A_KR <- D A_KR,  A_RR <- A_RR - A_RK D A_KR,
+// which keeps A symmetric, so only I <= J is computed and stored; after every block A holds
+// minus its inverse.  Two kernels per block: the panel (a CTA per tile of row K, each with its
+// own copy of D) and the rank-64 update of the other tiles.
+//
+// Bound: the serial chain of the nc pivots (a division and two barriers' worth of latency
+// each), then launches, then FP64 products (2 us for a 64^3 product on one SM).  As a sweep
+// over the full square in three kernels, the pivot block's inverse by one CTA with two barriers
+// per scalar step took 60 of 97 us per block, and the update twice the tiles in a second,
+// nearly empty wave.  Whole set-up: nc = 588 1.02 -> 0.51 ms, 1296 (Brick20 24^3) 2.50 -> 1.28,
+// 3072 (Q8 128) 7.06 -> 2.88; now 22 us the panel and 18 the update at nc = 1296.
+constexpr int kTS = 64;        // tile side and block size
+constexpr int kTT = kTS * kTS;
+constexpr int kTP = kTS + 4;   // shared row length: DMMA fragment loads on distinct banks
+constexpr size_t kSweepSmem = sizeof(double) * 2 * (size_t)kTS * kTP;
 
 __device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -634,112 +541,242 @@ __device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, do
                : "d"(a), "d"(b));
 }
 
-__global__ void __launch_bounds__(128)
-k_gj_update(int nc, int kb, int bs, double* __restrict__ A, const double* __restrict__ Pi,
-            const double* __restrict__ Rw, const double* __restrict__ Cold,
-            const double* __restrict__ Cn) {
+// index of tile (I, J), I <= J, among the nt (nt + 1) / 2 of the upper triangle
+__host__ __device__ inline int64_t tile_index(int nt, int I, int J) {
+  return (int64_t)I * nt - (int64_t)I * (I - 1) / 2 + (J - I);
+}
+
+// T = the upper-triangle tiles of the symmetric part of A, the identity beyond nc
+__global__ void __launch_bounds__(256)
+k_pack_tiles(int nc, const int2* __restrict__ ij, const double* __restrict__ A,
+             double* __restrict__ T) {
+  const int2 t = ij[blockIdx.x];
+  double* dst = T + (int64_t)blockIdx.x * kTT;
+  for (int e = threadIdx.x; e < kTT; e += 256) {
+    const int gi = t.x * kTS + e / kTS, gj = t.y * kTS + e % kTS;
+    dst[e] = (gi < nc && gj < nc)
+                 ? 0.5 * (A[(int64_t)gi * nc + gj] + A[(int64_t)gj * nc + gi])
+                 : gi == gj ? 1.0 : 0.0;
+  }
+}
+
+// M <- M^-1 (64 x 64, SPD) by 256 threads, each with a 4 x 4 piece in registers.  Two scalar
+// sweeps per barrier: their rows k, k + 1 go through shared memory, each thread does the second
+// pivot's elimination for itself, and with
+//   u, v = rows k and k + 1 (the latter after sweep k),  s = u / pivot1,  t = v / pivot2
+// every entry becomes x_ij - u_i s_j - v_i t_j, where for i or j in {k, k + 1} the old entry
+// drops out and u, v, s, t are replaced by the values that make this the swept row or column.
+__device__ __forceinline__ void invert_tile(double (*M)[kTP], double (&R)[2][2][kTS]) {
+  const int ti = threadIdx.x / 16, tj = threadIdx.x % 16;
+  double m[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) m[a][b] = M[4 * ti + a][4 * tj + b];
+#pragma unroll 1
+  for (int kt = 0; kt < kTS / 4; ++kt) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // pivots k = 4 kt + 2 h and k + 1; buffer h
+      const int k = 4 * kt + 2 * h;
+      if (ti == kt) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          R[h][0][4 * tj + b] = m[2 * h][b];
+          R[h][1][4 * tj + b] = m[2 * h + 1][b];
+        }
+      }
+      __syncthreads();
+      const double b01 = R[h][0][k + 1];
+      const double p1 = 1.0 / R[h][0][k];
+      const double l = b01 * p1;
+      const double p2 = 1.0 / (R[h][1][k + 1] - b01 * l);
+      double u[4], v[4], s[4], t[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        u[a] = R[h][0][4 * ti + a];
+        v[a] = R[h][1][4 * ti + a] - l * u[a];
+        const double uj = R[h][0][4 * tj + a];
+        s[a] = uj * p1;
+        t[a] = (R[h][1][4 * tj + a] - l * uj) * p2;
+      }
+      if (ti == kt) {
+        u[2 * h] = -1.0;
+        v[2 * h] = l;
+        u[2 * h + 1] = 0.0;
+        v[2 * h + 1] = -1.0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) m[2 * h][b] = m[2 * h + 1][b] = 0.0;
+      }
+      if (tj == kt) {
+        s[2 * h] = -p1;
+        t[2 * h] = l * p2;
+        s[2 * h + 1] = 0.0;
+        t[2 * h + 1] = -p2;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) m[a][2 * h] = m[a][2 * h + 1] = 0.0;
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) m[a][b] = (m[a][b] - u[a] * s[b]) - v[a] * t[b];
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) M[4 * ti + a][4 * tj + b] = -m[a][b];
+}
+
+// Panel of block K, CTA J: X = A_KJ (the transpose of the stored tile if J < K), W = D X.
+// Leaves X and W as 64 x 64 tiles in Xp[J], Wp[J] for the update, and W in the place of A_KJ
+// (-D for J = K).  Eight warps, a 16 x 32 piece of W each, as FP64 tensor-core products (per
+// lane one value A[g][t], one B[t][g], accumulators D[g][2t], D[g][2t + 1]; g = lane / 4,
+// t = lane % 4).
+__global__ void __launch_bounds__(256, 1)
+k_sweep_panel(int nt, int K, double* __restrict__ T, double* __restrict__ Xp,
+              double* __restrict__ Wp) {
   extern __shared__ __align__(16) double gsm[];
-  double (*sC)[kGU] = reinterpret_cast<double (*)[kGU]>(gsm);               // [row][u]
-  double (*sR)[kGU] = reinterpret_cast<double (*)[kGU]>(gsm + kGT * kGU);   // [u][col]
-  const int i0 = blockIdx.y * kGT, j0 = blockIdx.x * kGT;
+  double (*sD)[kTP] = reinterpret_cast<double (*)[kTP]>(gsm);              // [r][u]
+  double (*sX)[kTP] = reinterpret_cast<double (*)[kTP]>(gsm + kTS * kTP);  // [u][c]
+  __shared__ double R[2][2][kTS];
+  const int J = blockIdx.x, tid = threadIdx.x;
+  double* tK = T + tile_index(nt, K, K) * kTT;
+  double* tJ = T + (J < K ? tile_index(nt, J, K) : tile_index(nt, K, J)) * kTT;
+  // D's tile is overwritten by the CTA J = K: it leaves -D in Wp[K] instead, and the update
+  // kernel puts it in place
+  double d[kTT / 256], x[kTT / 256];
+#pragma unroll
+  for (int k = 0; k < kTT / 256; ++k) d[k] = __ldcg(tK + tid + 256 * k);
+  if (J != K) {
+#pragma unroll
+    for (int k = 0; k < kTT / 256; ++k) x[k] = __ldcg(tJ + tid + 256 * k);
+  }
+#pragma unroll
+  for (int k = 0; k < kTT / 256; ++k) {
+    const int e = tid + 256 * k;
+    sD[e / kTS][e % kTS] = d[k];
+    if (J > K) sX[e / kTS][e % kTS] = x[k];
+    if (J < K) sX[e % kTS][e / kTS] = x[k];
+  }
+  __syncthreads();
+  invert_tile(sD, R);
+  __syncthreads();
+  double* wp = Wp + (int64_t)J * kTT;
+  if (J == K) {
+    for (int e = tid; e < kTT; e += 256) wp[e] = -sD[e / kTS][e % kTS];
+    return;
+  }
+  const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  const int wr = (warp >> 1) * 16, wc = (warp & 1) * 32;
+  double acc[2][4][2] = {};
+#pragma unroll 4
+  for (int k0 = 0; k0 < kTS; k0 += 4) {
+    double a[2], b[4];
+#pragma unroll
+    for (int fm = 0; fm < 2; ++fm) a[fm] = sD[wr + fm * 8 + g][k0 + t4];
+#pragma unroll
+    for (int fn = 0; fn < 4; ++fn) b[fn] = sX[k0 + t4][wc + fn * 8 + g];
+#pragma unroll
+    for (int fm = 0; fm < 2; ++fm)
+#pragma unroll
+      for (int fn = 0; fn < 4; ++fn) dmma_m8n8k4(acc[fm][fn][0], acc[fm][fn][1], a[fm], b[fn]);
+  }
+  double* xp = Xp + (int64_t)J * kTT;
+  for (int e = tid; e < kTT; e += 256) xp[e] = sX[e / kTS][e % kTS];
+#pragma unroll
+  for (int fm = 0; fm < 2; ++fm)
+#pragma unroll
+    for (int fn = 0; fn < 4; ++fn) {
+      const int r = wr + fm * 8 + g, c = wc + fn * 8 + 2 * t4;
+      const double2 w = make_double2(acc[fm][fn][0], acc[fm][fn][1]);
+      *reinterpret_cast<double2*>(wp + r * kTS + c) = w;
+      if (J > K) {
+        *reinterpret_cast<double2*>(tJ + r * kTS + c) = w;
+      } else {
+        tJ[c * kTS + r] = w.x;
+        tJ[(c + 1) * kTS + r] = w.y;
+      }
+    }
+}
+
+// A_IJ -= X_I^T W_J for the tiles without block K (and -D into tile (K, K)): four warps, a
+// 32 x 32 quarter each, operands by 16-byte loads, all in flight at once.
+__global__ void __launch_bounds__(128)
+k_sweep_update(int K, const int2* __restrict__ ij, double* __restrict__ T,
+               const double* __restrict__ Xp, const double* __restrict__ Wp) {
+  extern __shared__ __align__(16) double gsm[];
+  double (*sX)[kTP] = reinterpret_cast<double (*)[kTP]>(gsm);              // [u][row]
+  double (*sW)[kTP] = reinterpret_cast<double (*)[kTP]>(gsm + kTS * kTP);  // [u][col]
+  const int2 t = ij[blockIdx.x];
+  double* tile = T + (int64_t)blockIdx.x * kTT;
   const int tid = threadIdx.x;
-  if (bs == kGJ && i0 + kGT <= nc && j0 + kGT <= nc && (nc & 1) == 0) {
-    // full interior tile, rows of Rw 16-byte aligned: 16-byte loads, all in flight at once
-    constexpr int P = kGT * kGJ / 2 / 128;   // double pairs per thread and operand
+  if (t.x == K || t.y == K) {
+    if (t.x == t.y)
+      for (int e = tid; e < kTT; e += 128) tile[e] = Wp[(int64_t)K * kTT + e];
+    return;
+  }
+  constexpr int P = kTT / 2 / 128;   // pairs per thread and operand
+  const double2* xs = reinterpret_cast<const double2*>(Xp + (int64_t)t.x * kTT);
+  const double2* ws = reinterpret_cast<const double2*>(Wp + (int64_t)t.y * kTT);
+  {
     double2 c[P], r[P];
 #pragma unroll
     for (int k = 0; k < P; ++k) {
-      const int e = tid + 128 * k;            // pair index: row e / 32, pair e % 32
-      c[k] = __ldcg(reinterpret_cast<const double2*>(Cold + (int64_t)(i0 + e / 32) * kGJ) + e % 32);
-      r[k] = __ldcg(reinterpret_cast<const double2*>(Rw + (int64_t)(e / 32) * nc + j0) + e % 32);
+      c[k] = __ldcg(xs + tid + 128 * k);
+      r[k] = __ldcg(ws + tid + 128 * k);
     }
 #pragma unroll
     for (int k = 0; k < P; ++k) {
-      const int e = tid + 128 * k;
-      sC[e / 32][2 * (e % 32)] = c[k].x;
-      sC[e / 32][2 * (e % 32) + 1] = c[k].y;
-      sR[e / 32][2 * (e % 32)] = r[k].x;
-      sR[e / 32][2 * (e % 32) + 1] = r[k].y;
-    }
-  } else {
-    for (int e = tid; e < kGT * kGJ; e += 128) {
-      const int r = e / kGJ, u = e % kGJ;
-      sC[r][u] = (i0 + r < nc && u < bs) ? Cold[(int64_t)(i0 + r) * kGJ + u] : 0.0;
-      const int u2 = e / kGT, c2 = e % kGT;
-      sR[u2][c2] = (j0 + c2 < nc && u2 < bs) ? Rw[(int64_t)u2 * nc + j0 + c2] : 0.0;
+      const int e = tid + 128 * k;  // pair index: row e / 32, pair e % 32
+      *reinterpret_cast<double2*>(&sX[e / 32][2 * (e % 32)]) = c[k];
+      *reinterpret_cast<double2*>(&sW[e / 32][2 * (e % 32)]) = r[k];
     }
   }
   __syncthreads();
-  const int warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t4 = lane & 3;
+  const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
   const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32;
-  double acc[4][4][2];
-#pragma unroll
-  for (int fm = 0; fm < 4; ++fm)
-#pragma unroll
-    for (int fn = 0; fn < 4; ++fn) acc[fm][fn][0] = acc[fm][fn][1] = 0.0;
+  double acc[4][4][2] = {};
 #pragma unroll 4
-  for (int k0 = 0; k0 < kGJ; k0 += 4) {
+  for (int k0 = 0; k0 < kTS; k0 += 4) {
     double a[4], b[4];
 #pragma unroll
-    for (int fm = 0; fm < 4; ++fm) a[fm] = sC[wr + fm * 8 + g][k0 + t4];
+    for (int fm = 0; fm < 4; ++fm) a[fm] = sX[k0 + t4][wr + fm * 8 + g];
 #pragma unroll
-    for (int fn = 0; fn < 4; ++fn) b[fn] = sR[k0 + t4][wc + fn * 8 + g];
+    for (int fn = 0; fn < 4; ++fn) b[fn] = sW[k0 + t4][wc + fn * 8 + g];
 #pragma unroll
     for (int fm = 0; fm < 4; ++fm)
 #pragma unroll
       for (int fn = 0; fn < 4; ++fn) dmma_m8n8k4(acc[fm][fn][0], acc[fm][fn][1], a[fm], b[fn]);
   }
-  const bool plain = i0 + kGT <= nc && j0 + kGT <= nc && (nc & 1) == 0 &&
-                     (kb + bs <= i0 || kb >= i0 + kGT) && (kb + bs <= j0 || kb >= j0 + kGT);
-  if (plain) {
-    // no pivot row or column in the tile: 16-byte read-modify-writes of the entry pairs
-#pragma unroll
-    for (int fm = 0; fm < 4; ++fm) {
-      double2* row = reinterpret_cast<double2*>(A + (int64_t)(i0 + wr + fm * 8 + g) * nc + j0 + wc);
-#pragma unroll
-      for (int fn = 0; fn < 4; ++fn) {
-        double2 v = row[fn * 4 + t4];
-        v.x -= acc[fm][fn][0];
-        v.y -= acc[fm][fn][1];
-        row[fn * 4 + t4] = v;
-      }
-    }
-    return;
-  }
 #pragma unroll
   for (int fm = 0; fm < 4; ++fm) {
-    const int i = i0 + wr + fm * 8 + g;
-    if (i >= nc) continue;
-    const bool ip = i >= kb && i < kb + bs;
+    double2* row = reinterpret_cast<double2*>(tile + (wr + fm * 8 + g) * kTS + wc);
 #pragma unroll
-    for (int fn = 0; fn < 4; ++fn)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int j = j0 + wc + fn * 8 + 2 * t4 + h;
-        if (j >= nc) continue;
-        const bool jp = j >= kb && j < kb + bs;
-        double* dst = A + (int64_t)i * nc + j;
-        if (ip && jp) *dst = Pi[(i - kb) * kGJ + (j - kb)];
-        else if (ip) *dst = Rw[(int64_t)(i - kb) * nc + j];
-        else if (jp) *dst = Cn[(int64_t)i * kGJ + (j - kb)];
-        else *dst -= acc[fm][fn][h];
-      }
+    for (int fn = 0; fn < 4; ++fn) {
+      double2 v = row[fn * 4 + t4];
+      v.x -= acc[fm][fn][0];
+      v.y -= acc[fm][fn][1];
+      row[fn * 4 + t4] = v;
+    }
   }
 }
 
-// Upper-triangle tiles (I <= J) of the symmetrised inverse, zero beyond nc.
-constexpr int kTS = 64;
-__global__ void k_pack_tiles(int nc, const int2* __restrict__ ij, const double* __restrict__ A,
-                             double* __restrict__ T) {
+// T <- the inverse from the swept tiles (minus it): negated, diagonal tiles symmetrised, zero
+// beyond nc
+__global__ void __launch_bounds__(256)
+k_sweep_finish(int nc, const int2* __restrict__ ij, double* __restrict__ T) {
   const int2 t = ij[blockIdx.x];
-  double* dst = T + (int64_t)blockIdx.x * kTS * kTS;
-  for (int e = threadIdx.x; e < kTS * kTS; e += blockDim.x) {
-    const int gi = t.x * kTS + e / kTS, gj = t.y * kTS + e % kTS;
-    dst[e] = (gi < nc && gj < nc)
-                 ? 0.5 * (A[(int64_t)gi * nc + gj] + A[(int64_t)gj * nc + gi])
-                 : 0.0;
+  double* tile = T + (int64_t)blockIdx.x * kTT;
+  double v[kTT / 256];
+#pragma unroll
+  for (int k = 0; k < kTT / 256; ++k) {
+    const int e = threadIdx.x + 256 * k, r = e / kTS, c = e % kTS;
+    const double x = t.x == t.y ? 0.5 * (tile[e] + tile[c * kTS + r]) : tile[e];
+    v[k] = t.x * kTS + r < nc && t.y * kTS + c < nc ? -x : 0.0;
   }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kTT / 256; ++k) tile[threadIdx.x + 256 * k] = v[k];
 }
 
 // rc = P^T r (and zc = 0 for the coarse product): block per aggregate over its node list
@@ -1172,12 +1209,11 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
   C->dim = dim; C->nm = nm; C->na = na; C->nc = nc; C->s = side;
   for (int c = 0; c < 3; ++c) { C->lo[c] = g.lo[c]; C->nb[c] = g.nb[c]; }
   double* d_Ac = nullptr;
-  double *d_pi = nullptr, *d_rw = nullptr, *d_cold = nullptr, *d_cn = nullptr,
-         *d_dmax = nullptr;
+  double *d_xp = nullptr, *d_wp = nullptr, *d_dmax = nullptr;
   double4* d_rec = nullptr;   // per-node records of the slice coarse kernel
   auto cleanup2 = [&]() {
     cleanup();
-    gf_pfree(ctx, d_Ac); gf_pfree(ctx, d_pi); gf_pfree(ctx, d_rw); gf_pfree(ctx, d_cold); gf_pfree(ctx, d_cn);
+    gf_pfree(ctx, d_Ac); gf_pfree(ctx, d_xp); gf_pfree(ctx, d_wp);
     gf_pfree(ctx, d_dmax); gf_pfree(ctx, d_rec);
   };
   if ((st = gf_palloc(ctx, &C->node_agg, (size_t)nnodes)) != GF_OK ||
@@ -1190,10 +1226,8 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
       (st = gf_palloc(ctx, &C->rc, (size_t)ld * C->parts)) != GF_OK ||
       (st = gf_palloc(ctx, &C->zc, (size_t)ld)) != GF_OK ||
       (st = gf_palloc(ctx, &d_Ac, (size_t)nc * nc)) != GF_OK ||
-      (st = gf_palloc(ctx, &d_pi, (size_t)kGJ * kGJ)) != GF_OK ||
-      (st = gf_palloc(ctx, &d_rw, (size_t)kGJ * nc)) != GF_OK ||
-      (st = gf_palloc(ctx, &d_cold, (size_t)kGJ * nc)) != GF_OK ||
-      (st = gf_palloc(ctx, &d_cn, (size_t)kGJ * nc)) != GF_OK ||
+      (st = gf_palloc(ctx, &d_xp, (size_t)nt * kTT)) != GF_OK ||
+      (st = gf_palloc(ctx, &d_wp, (size_t)nt * kTT)) != GF_OK ||
       (st = gf_palloc(ctx, &d_dmax, 1)) != GF_OK) {
     cleanup2();
     return st;
@@ -1272,17 +1306,7 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
   k_diag_max<<<1, kCT, 0, s>>>(nc, d_Ac, d_dmax);
   k_regularise<<<gf_blocks(nc, kCT), kCT, 0, s>>>(nc, d_dmax, 1e-10, d_Ac);
   ctx->launches += 8;
-  // blocked Gauss-Jordan inverse
-  const dim3 gp((nc + kGT - 1) / kGT, 2), gu((nc + kGT - 1) / kGT, (nc + kGT - 1) / kGT);
-  GF_CUDA(ctx, gf_smem_attr(k_gj_panels, kGJSmem));
-  GF_CUDA(ctx, gf_smem_attr(k_gj_update, kGJUpdateSmem));
-  for (int kb = 0; kb < nc; kb += kGJ) {
-    const int bs = std::min(kGJ, nc - kb);
-    k_gj_pivot<<<1, dim3(kGJ, kGJRows), 0, s>>>(nc, kb, bs, d_Ac, d_pi);
-    k_gj_panels<<<gp, 256, kGJSmem, s>>>(nc, kb, bs, d_Ac, d_pi, d_rw, d_cold, d_cn);
-    k_gj_update<<<gu, 128, kGJUpdateSmem, s>>>(nc, kb, bs, d_Ac, d_pi, d_rw, d_cold, d_cn);
-    ctx->launches += 3;
-  }
+  // its inverse, in the tiles of the coarse product
   std::vector<int2> hij;
   hij.reserve(ntiles);
   for (int I = 0; I < nt; ++I)
@@ -1290,6 +1314,14 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
   GF_CUDA(ctx, cudaMemcpyAsync(C->tile_ij, hij.data(), sizeof(int2) * ntiles,
                                cudaMemcpyHostToDevice, s));
   k_pack_tiles<<<ntiles, 256, 0, s>>>(nc, C->tile_ij, d_Ac, C->ainv);
+  GF_CUDA(ctx, gf_smem_attr(k_sweep_panel, kSweepSmem));
+  GF_CUDA(ctx, gf_smem_attr(k_sweep_update, kSweepSmem));
+  for (int K = 0; K < nt; ++K) {
+    k_sweep_panel<<<nt, 256, kSweepSmem, s>>>(nt, K, C->ainv, d_xp, d_wp);
+    k_sweep_update<<<ntiles, 128, kSweepSmem, s>>>(K, C->tile_ij, C->ainv, d_xp, d_wp);
+  }
+  k_sweep_finish<<<ntiles, 256, 0, s>>>(nc, C->tile_ij, C->ainv);
+  ctx->launches += 1 + 2 * (int64_t)nt;
   cudaMemsetAsync(C->rc, 0, sizeof(double) * ld * C->parts, s);  // the tails beyond nc stay zero
   cudaMemsetAsync(C->zc, 0, sizeof(double) * ld, s);
   ctx->launches++;
