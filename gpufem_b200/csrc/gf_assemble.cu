@@ -17,7 +17,7 @@
 // each writes block (i,j) and its transpose (j,i).
 //
 // CTA = a tile of TE elements of one colour (or any elements for the atomic
-// scatter), 256 threads:
+// scatter; Brick20 takes gf_assemble_b20.cu there), 256 threads:
 //   phase 1  thread per (element, Gauss point): J, detJ, J^-1, g = J^-1 dN/dxi
 //            into shared memory G[gp][node][comp][elem]; for the FP32 path an
 //            element whose max/min |detJ| over its Gauss points exceeds 10 gets
@@ -31,6 +31,8 @@
 #include <algorithm>
 
 #include "gf_elem.cuh"
+
+gf_status gf_assemble_b20(gf_ctx* ctx, int dtype, const AsmTables* d_tab);
 
 namespace {
 
@@ -245,25 +247,27 @@ gf_status launch_et_ng(gf_ctx* ctx, int scatter, const AsmTables* d_tab, TC* K) 
   constexpr size_t sm = smem_bytes<ET, TC>(TE, ngp);
   const double* coords = ctx->d_coords64;
   const TC* Eel = sizeof(TC) == 8 ? (const TC*)ctx->d_Eel : (const TC*)ctx->d_Eel32;
-  auto kc = k_assemble<ET, TC, false, NG1>;
-  auto ka = k_assemble<ET, TC, true, NG1>;
-  GF_CUDA(ctx, gf_smem_attr(kc, (int)sm));
-  GF_CUDA(ctx, gf_smem_attr(ka, (int)sm));
-  if (scatter == GF_SCATTER_ATOMIC) {
-    const int count = ctx->nelem;
-    ka<<<(count + TE - 1) / TE, kThreads, sm, ctx->stream>>>(
-        ctx->d_allperm, count, ctx->d_conn, coords, Eel, ctx->d_slotmap, ctx->nelem, ctx->n,
-        d_tab, TC(ctx->lam1), TC(ctx->mu1), K);
-    GF_LAUNCH_CHECK(ctx, "k_assemble(atomic)");
-  } else {
-    for (int c = 0; c < ctx->ncolors; ++c) {
-      const int c0 = ctx->color_off[c], count = ctx->color_off[c + 1] - c0;
-      if (count == 0) continue;
-      kc<<<(count + TE - 1) / TE, kThreads, sm, ctx->stream>>>(
-          ctx->d_perm + c0, count, ctx->d_conn, coords, Eel, ctx->d_slotmap, ctx->nelem,
-          ctx->n, d_tab, TC(ctx->lam1), TC(ctx->mu1), K);
-      GF_LAUNCH_CHECK(ctx, "k_assemble(colour)");
+  if constexpr (ET != GF_BRICK20) {  // Brick20: gf_assemble_b20.cu
+    if (scatter == GF_SCATTER_ATOMIC) {
+      auto ka = k_assemble<ET, TC, true, NG1>;
+      GF_CUDA(ctx, gf_smem_attr(ka, (int)sm));
+      const int count = ctx->nelem;
+      ka<<<(count + TE - 1) / TE, kThreads, sm, ctx->stream>>>(
+          ctx->d_allperm, count, ctx->d_conn, coords, Eel, ctx->d_slotmap, ctx->nelem, ctx->n,
+          d_tab, TC(ctx->lam1), TC(ctx->mu1), K);
+      GF_LAUNCH_CHECK(ctx, "k_assemble(atomic)");
+      return GF_OK;
     }
+  }
+  auto kc = k_assemble<ET, TC, false, NG1>;
+  GF_CUDA(ctx, gf_smem_attr(kc, (int)sm));
+  for (int c = 0; c < ctx->ncolors; ++c) {
+    const int c0 = ctx->color_off[c], count = ctx->color_off[c + 1] - c0;
+    if (count == 0) continue;
+    kc<<<(count + TE - 1) / TE, kThreads, sm, ctx->stream>>>(
+        ctx->d_perm + c0, count, ctx->d_conn, coords, Eel, ctx->d_slotmap, ctx->nelem, ctx->n,
+        d_tab, TC(ctx->lam1), TC(ctx->mu1), K);
+    GF_LAUNCH_CHECK(ctx, "k_assemble(colour)");
   }
   return GF_OK;
 }
@@ -276,6 +280,8 @@ gf_status launch_et(gf_ctx* ctx, int scatter, const AsmTables* d_tab, TC* K) {
 
 template <typename TC>
 gf_status launch_dispatch(gf_ctx* ctx, int scatter, const AsmTables* d_tab, TC* K) {
+  if (ctx->elem_type == GF_BRICK20 && scatter == GF_SCATTER_ATOMIC)
+    return gf_assemble_b20(ctx, sizeof(TC) == 8 ? GF_F64 : GF_F32, d_tab);
   switch (ctx->elem_type) {
     case GF_Q4: return launch_et<GF_Q4, TC>(ctx, scatter, d_tab, K);
     case GF_Q8: return launch_et<GF_Q8, TC>(ctx, scatter, d_tab, K);
@@ -345,7 +351,10 @@ gf_status gf_assemble_launch(gf_ctx* ctx, int dtype, int scatter, int engine) {
       ctx->gram_bytes = need;
     }
   }
-  if (scatter != GF_SCATTER_OWNER && (st = gf_slotmap_ensure(ctx)) != GF_OK) return st;
+  const bool b20 = !mma && scatter == GF_SCATTER_ATOMIC && ctx->elem_type == GF_BRICK20;
+  if (scatter != GF_SCATTER_OWNER &&
+      (st = b20 ? gf_einc_ensure(ctx) : gf_slotmap_ensure(ctx)) != GF_OK)
+    return st;
   cudaEventRecord(ctx->ev0, ctx->stream);
   if (mma && scatter == GF_SCATTER_OWNER) {
     // tensor cores: every element's Gram matrix to HBM; owner gather: K written once

@@ -219,6 +219,7 @@ struct gf_ctx {
   int32_t* d_inc = nullptr;
   uint8_t* d_inc_loc = nullptr;   // local index of the node within each incident element
   uint16_t* d_inc_slot = nullptr; // [incidence][nen]: neighbour position of each element node
+  int32_t* d_einc = nullptr;      // [nelem][nen] incidence of each element node (Brick20 atomic)
   int maxval = 0;                 // max elements sharing one node
   void* d_geo = nullptr;          // owner scatter: J^-1, w detJ per (element, Gauss point)
   size_t geo_bytes = 0;
@@ -373,6 +374,7 @@ inline int gf_blocks(int64_t work, int threads) {
 // internal entry points across translation units
 gf_status gf_pattern_build(gf_ctx* ctx);
 gf_status gf_slotmap_ensure(gf_ctx* ctx);
+gf_status gf_einc_ensure(gf_ctx* ctx);
 gf_status gf_color_build(gf_ctx* ctx, const int32_t* user_colors);
 bool gf_assemble_node_fits(const gf_ctx* ctx, int dtype);
 gf_status gf_geo_buffer(gf_ctx* ctx, size_t bytes);

@@ -513,6 +513,12 @@ __global__ void k_slotmap(int nelem, int nen, const int32_t* __restrict__ conn,
   for (int j = 0; j < nen; ++j) slotmap[(int64_t)(i * nen + j) * nelem + e] = __ldg(src + j);
 }
 
+__global__ void k_einc(int64_t total, int nen, const int32_t* __restrict__ inc,
+                       const uint8_t* __restrict__ inc_loc, int32_t* __restrict__ einc) {
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (q < total) einc[(int64_t)inc[q] * nen + inc_loc[q]] = (int32_t)q;
+}
+
 __global__ void k_diagpos(int nnodes, const int32_t* __restrict__ adj_off,
                           const int32_t* __restrict__ adj, int32_t* __restrict__ diagpos) {
   int a = blockIdx.x * blockDim.x + threadIdx.x;
@@ -784,6 +790,20 @@ gf_status gf_slotmap_ensure(gf_ctx* ctx) {
     return e != cudaSuccess ? gf_cuda_fail(ctx, e, "slot map")
                             : gf_fail(ctx, GF_ERR_CUDA, "slot map lookup failed");
   }
+  return GF_OK;
+}
+
+// Incidence of every element node (the inverse of inc / inc_loc), through which the Brick20
+// reductions find their slots; built on the first assembly that needs it.
+gf_status gf_einc_ensure(gf_ctx* ctx) {
+  if (ctx->d_einc) return GF_OK;
+  if (!ctx->has_pattern) return gf_fail(ctx, GF_ERR_STATE, "no pattern");
+  const int64_t total = (int64_t)ctx->nelem * ctx->nen;
+  gf_status st = gf_palloc(ctx, &ctx->d_einc, (size_t)total);
+  if (st != GF_OK) return st;
+  k_einc<<<gf_blocks(total, 256), 256, 0, ctx->stream>>>(total, ctx->nen, ctx->d_inc,
+                                                         ctx->d_inc_loc, ctx->d_einc);
+  GF_LAUNCH_CHECK(ctx, "k_einc");
   return GF_OK;
 }
 
