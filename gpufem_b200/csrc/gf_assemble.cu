@@ -319,7 +319,8 @@ gf_status gf_asm_tables(gf_ctx* ctx, const AsmTables** out) {
   AsmTables* d = nullptr;
   gf_status st = gf_alloc(ctx, &d, 1);
   if (st != GF_OK) return st;
-  GF_CUDA(ctx, cudaMemcpy(d, &h, sizeof(AsmTables), cudaMemcpyHostToDevice));
+  GF_CUDA(ctx, cudaMemcpyAsync(d, &h, sizeof(AsmTables), cudaMemcpyHostToDevice, ctx->stream));
+  GF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->d_asmtab = d;
   *out = d;
   return GF_OK;

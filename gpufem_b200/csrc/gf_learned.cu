@@ -1082,7 +1082,7 @@ GF_API gf_status gf_lp_init(gf_ctx* ctx, int32_t dim, uint64_t seed) {
   if ((st = lp_alloc(ctx, &s->v, (size_t)P)) != GF_OK) return st;
   if ((st = lp_alloc(ctx, &s->sc, 1)) != GF_OK) return st;
   if ((st = lp_alloc(ctx, &s->err, 1)) != GF_OK) return st;
-  GF_CUDA(ctx, cudaMemset(s->err, 0, sizeof(int)));
+  GF_CUDA(ctx, cudaMemsetAsync(s->err, 0, sizeof(int), ctx->stream));
   if ((st = lp_mm_setup(ctx, dim)) != GF_OK) return st;
   // He-style init for hidden layers; output layer zero (untrained = Jacobi)
   std::vector<float> w(P, 0.f);
@@ -1096,9 +1096,12 @@ GF_API gf_status gf_lp_init(gf_ctx* ctx, int32_t dim, uint64_t seed) {
       w[o.Ws[l] + k] = nd(rng) * std::sqrt(1.f / H);
       w[o.Wn[l] + k] = nd(rng) * std::sqrt(1.f / H);
     }
-  GF_CUDA(ctx, cudaMemcpy(s->w, w.data(), sizeof(float) * P, cudaMemcpyHostToDevice));
-  GF_CUDA(ctx, cudaMemset(s->m, 0, sizeof(float) * P));
-  GF_CUDA(ctx, cudaMemset(s->v, 0, sizeof(float) * P));
+  // on the context's stream: it does not wait for the default stream, and a copy of pageable
+  // memory may return before it has reached the device
+  GF_CUDA(ctx, cudaMemcpyAsync(s->w, w.data(), sizeof(float) * P, cudaMemcpyHostToDevice,
+                               ctx->stream));
+  GF_CUDA(ctx, cudaMemsetAsync(s->m, 0, sizeof(float) * P, ctx->stream));
+  GF_CUDA(ctx, cudaMemsetAsync(s->v, 0, sizeof(float) * P, ctx->stream));
   k_lp_to_bf16<<<gf_blocks(P, kLT), kLT, 0, ctx->stream>>>(P, s->w, s->wb);
   GF_LAUNCH_CHECK(ctx, "k_lp_to_bf16");
   GF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1122,7 +1125,7 @@ GF_API gf_status gf_lp_set_weights(gf_ctx* ctx, const float* w) {
   const int64_t P = s->off.total;
   for (int64_t k = 0; k < P; ++k)
     if (!std::isfinite(w[k])) return gf_fail(ctx, GF_ERR_INVALID_ARG, "non-finite weight %lld", (long long)k);
-  GF_CUDA(ctx, cudaMemcpy(s->w, w, sizeof(float) * P, cudaMemcpyHostToDevice));
+  GF_CUDA(ctx, cudaMemcpyAsync(s->w, w, sizeof(float) * P, cudaMemcpyHostToDevice, ctx->stream));
   k_lp_to_bf16<<<gf_blocks(P, kLT), kLT, 0, ctx->stream>>>(P, s->w, s->wb);
   GF_LAUNCH_CHECK(ctx, "k_lp_to_bf16");
   GF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

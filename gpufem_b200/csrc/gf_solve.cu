@@ -1829,9 +1829,12 @@ extern "C" GF_API gf_status gf_dist_set_halo(gf_ctx* ctx, int32_t n_owned, int32
   if ((st = gf_alloc(ctx, &d->d_vec, (size_t)4 * n_owned + 2 * (size_t)n)) != GF_OK) return st;
   if ((st = gf_alloc(ctx, &d->d_sc, 1)) != GF_OK) return st;
   if (n_send)
-    GF_CUDA(ctx, cudaMemcpy(d->d_send, send_dofs, sizeof(int32_t) * n_send, cudaMemcpyHostToDevice));
+    GF_CUDA(ctx, cudaMemcpyAsync(d->d_send, send_dofs, sizeof(int32_t) * n_send,
+                                 cudaMemcpyHostToDevice, ctx->stream));
   if (n_recv)
-    GF_CUDA(ctx, cudaMemcpy(d->d_recv, recv_dofs, sizeof(int32_t) * n_recv, cudaMemcpyHostToDevice));
+    GF_CUDA(ctx, cudaMemcpyAsync(d->d_recv, recv_dofs, sizeof(int32_t) * n_recv,
+                                 cudaMemcpyHostToDevice, ctx->stream));
+  GF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return GF_OK;
 }
 

@@ -51,3 +51,21 @@ def test_matrix_changes_reach_the_next_application(dtypes):
     for a, b in zip(again, want):
         assert np.linalg.norm(a - b) <= 1e-5 * np.linalg.norm(b)
     assert np.linalg.norm(want[0] - want[1]) > 1e-3 * np.linalg.norm(want[0])
+
+
+def test_set_weights_reach_the_next_application():
+    """New weights, and the first ones again, many times over."""
+    m, ctx = context(1.0, (_lib.GF_F64,))
+    r = np.random.default_rng(0).normal(size=m.ndof).astype(np.float32)
+    P = ctx.lp_num_params(3)
+    ws = [np.random.default_rng(k).normal(scale=0.2, size=P).astype(np.float32) for k in (5, 6)]
+    want = []
+    for w in ws:
+        for _ in range(3):
+            ctx.lp_set_weights(w)
+        want.append(ctx.lp_apply(r))
+    assert np.linalg.norm(want[0] - want[1]) > 1e-3 * np.linalg.norm(want[0])
+    for k in range(100):
+        ctx.lp_set_weights(ws[k % 2])
+        z = ctx.lp_apply(r)
+        assert np.linalg.norm(z - want[k % 2]) <= 1e-5 * np.linalg.norm(want[k % 2]), k
