@@ -48,6 +48,8 @@ GF_API gf_status gf_create(gf_ctx** out, int32_t device) {
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess ||
+      cudaEventCreate(&ctx->eva0) != cudaSuccess || cudaEventCreate(&ctx->eva1) != cudaSuccess ||
+      cudaEventCreate(&ctx->evs0) != cudaSuccess || cudaEventCreate(&ctx->evs1) != cudaSuccess ||
       cudaEventCreate(&ctx->evm) != cudaSuccess) {
     cudaGetLastError();
     delete ctx;
@@ -76,7 +78,11 @@ GF_API gf_status gf_destroy(gf_ctx* ctx) {
   gf_pool_clear(ctx);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
+  if (ctx->eva0) cudaEventDestroy(ctx->eva0);
+  if (ctx->eva1) cudaEventDestroy(ctx->eva1);
   if (ctx->evm) cudaEventDestroy(ctx->evm);
+  if (ctx->evs0) cudaEventDestroy(ctx->evs0);
+  if (ctx->evs1) cudaEventDestroy(ctx->evs1);
   if (ctx->ev_dl) cudaEventDestroy(ctx->ev_dl);
   if (ctx->h_adj_stage) cudaFreeHost(ctx->h_adj_stage);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -85,14 +91,22 @@ GF_API gf_status gf_destroy(gf_ctx* ctx) {
 }
 
 GF_API const char* gf_last_error(const gf_ctx* ctx) { return ctx ? ctx->err.c_str() : "null context"; }
-GF_API double gf_last_device_seconds(const gf_ctx* ctx) { return ctx ? ctx->last_seconds : 0.0; }
+GF_API double gf_last_device_seconds(const gf_ctx* ctx) {
+  if (!ctx) return 0.0;
+  return ctx->timed0 ? gf_elapsed(ctx->timed0, ctx->timed1) : ctx->last_seconds;
+}
 GF_API int64_t gf_kernel_launches(const gf_ctx* ctx) { return ctx ? ctx->launches : 0; }
 
 GF_API gf_status gf_last_assembly_split(const gf_ctx* ctx, double* geometry_seconds,
                                         double* scatter_seconds) {
   if (!ctx) return GF_ERR_INVALID_ARG;
-  if (geometry_seconds) *geometry_seconds = ctx->last_split[0];
-  if (scatter_seconds) *scatter_seconds = ctx->last_split[1];
+  double geo = 0.0, scatter = 0.0;
+  if (ctx->has_split) {
+    if (ctx->split_owner) geo = gf_elapsed(ctx->eva0, ctx->evm);
+    scatter = gf_elapsed(ctx->split_owner ? ctx->evm : ctx->eva0, ctx->eva1);
+  }
+  if (geometry_seconds) *geometry_seconds = geo;
+  if (scatter_seconds) *scatter_seconds = scatter;
   return GF_OK;
 }
 
@@ -521,8 +535,13 @@ GF_API gf_status gf_assemble(gf_ctx* ctx, int32_t dtype, int32_t scatter, int32_
   if (!ctx->has_pattern && (st = gf_pattern_build(ctx)) != GF_OK) return st;
   // the fastest measured schedule (B200): Brick8 128^3 FP32 1.56 ms by owners, 3.82 ms with
   // atomics; Brick20 64^3 FP32 3.10 ms with atomics, 7.94 ms by owners
+  // small FP64 Brick8 meshes: an SM gets two warps of owners or fewer, each a serial chain of
+  // FP64 sums, 42 us at 8^3 and 48 at 21^3 against 27 and 46 with atomics (22^3: 48 and 57)
+  const bool b8_small = ctx->elem_type == GF_BRICK8 && dtype == GF_F64 &&
+                        ctx->nnodes <= 76 * (int64_t)ctx->sm_count;
   if (scatter == GF_SCATTER_AUTO)
-    scatter = ctx->dim == 2 || engine == GF_ENGINE_TF32_MMA || gf_assemble_node_fits(ctx, dtype)
+    scatter = ctx->dim == 2 || engine == GF_ENGINE_TF32_MMA ||
+                      (gf_assemble_node_fits(ctx, dtype) && !b8_small)
                   ? GF_SCATTER_OWNER
                   : GF_SCATTER_ATOMIC;
   if (scatter == GF_SCATTER_COLOR && ctx->ncolors == 0 &&

@@ -356,7 +356,8 @@ gf_status gf_assemble_launch(gf_ctx* ctx, int dtype, int scatter, int engine) {
   if (scatter != GF_SCATTER_OWNER &&
       (st = b20 ? gf_einc_ensure(ctx) : gf_slotmap_ensure(ctx)) != GF_OK)
     return st;
-  cudaEventRecord(ctx->ev0, ctx->stream);
+  ctx->has_split = false;
+  ctx->time_begin(ctx->eva0);
   if (mma && scatter == GF_SCATTER_OWNER) {
     // tensor cores: every element's Gram matrix to HBM; owner gather: K written once
     st = gf_assemble_tc(ctx, scatter, d_tab, ctx->d_gram, ctx->d_asm_err);
@@ -374,7 +375,7 @@ gf_status gf_assemble_launch(gf_ctx* ctx, int dtype, int scatter, int engine) {
     st = mma ? gf_assemble_tc(ctx, scatter, d_tab, ctx->d_K32, ctx->d_asm_err)
              : launch_dispatch<float>(ctx, scatter, d_tab, ctx->d_K32);
   }
-  cudaEventRecord(ctx->ev1, ctx->stream);
+  cudaEventRecord(ctx->eva1, ctx->stream);
   cudaError_t e = cudaStreamSynchronize(ctx->stream);
   if (st != GF_OK) return st;
   if (e != cudaSuccess) return gf_cuda_fail(ctx, e, "assembly");
@@ -384,19 +385,9 @@ gf_status gf_assemble_launch(gf_ctx* ctx, int dtype, int scatter, int engine) {
     if (herr)
       return gf_fail(ctx, GF_ERR_CUDA, "tensor-core assembly: an MMA completion wait timed out");
   }
-  float ms = 0.f;
-  cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-  ctx->last_seconds = ms * 1e-3;
-  if (scatter == GF_SCATTER_OWNER) {
-    float m0 = 0.f, m1 = 0.f;
-    cudaEventElapsedTime(&m0, ctx->ev0, ctx->evm);
-    cudaEventElapsedTime(&m1, ctx->evm, ctx->ev1);
-    ctx->last_split[0] = m0 * 1e-3;
-    ctx->last_split[1] = m1 * 1e-3;
-  } else {
-    ctx->last_split[0] = 0.0;
-    ctx->last_split[1] = ms * 1e-3;
-  }
+  ctx->time_end(ctx->eva0, ctx->eva1);
+  ctx->has_split = true;
+  ctx->split_owner = scatter == GF_SCATTER_OWNER;
   if (dtype == GF_F64) { ctx->has64 = true; ctx->kver64++; } else { ctx->has32 = true; ctx->kver32++; }
   ctx->bc_mode_applied = -1;
   return GF_OK;

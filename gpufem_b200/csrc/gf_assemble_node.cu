@@ -652,9 +652,12 @@ gf_status gf_geo_buffer(gf_ctx* ctx, size_t bytes) {
 }
 
 // Whether this file's kernels take the mesh: Q4, Q8 and Brick8 whose rows fit their tiles (32
-// nodes; 28 in FP64 Brick8) within 112 KB, two CTAs per SM.
+// nodes; 28 in FP64 Brick8) within 112 KB, two CTAs per SM.  FP64 Brick8 meshes of less than a
+// warp per SM stay with a thread per (node, element): 36 against 42 us at 8^3 (16^3: 48 and 45).
 bool gf_assemble_node_fits(const gf_ctx* ctx, int dtype) {
   if (ctx->elem_type == GF_BRICK20) return false;
+  if (ctx->elem_type == GF_BRICK8 && dtype == GF_F64 && ctx->nnodes <= 24 * (int64_t)ctx->sm_count)
+    return false;
   const size_t es = dtype == GF_F64 ? 8 : 4;
   const size_t rows = ctx->dim == 2 ? 64 : 3 * (dtype == GF_F64 ? b8_nodes<double>() : b8_nodes<float>());
   return es * (rows * (size_t)ctx->W + 27 * 8 * 4) + 4 * 1024 <= 112 * 1024;

@@ -165,10 +165,28 @@ struct gf_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t eva0 = nullptr, eva1 = nullptr;  // around the last assembly
   cudaEvent_t evm = nullptr;            // between the two kernels of an owner assembly
-  double last_split[2] = {0.0, 0.0};    // last assembly: geometry, scatter kernel seconds
+  cudaEvent_t evs0 = nullptr, evs1 = nullptr;  // around the last gf_spmv or gf_lp_apply
+  bool has_split = false, split_owner = false;  // eva0, eva1 (and evm) hold an assembly
   std::string err;
+  // Device time of the last timed call: last_seconds, or between two events whose elapsed time is
+  // taken when asked for (each such query costs a short call 3 us).
   double last_seconds = 0.0;
+  cudaEvent_t timed0 = nullptr, timed1 = nullptr;
+  void set_seconds(double s) {
+    last_seconds = s;
+    timed0 = timed1 = nullptr;
+  }
+  // Around a short timed call: its events hold nothing until it has succeeded.
+  void time_begin(cudaEvent_t e0) {
+    if (timed0 == e0) set_seconds(0.0);
+    cudaEventRecord(e0, stream);
+  }
+  void time_end(cudaEvent_t e0, cudaEvent_t e1) {
+    timed0 = e0;
+    timed1 = e1;
+  }
   int64_t launches = 0;
   int sm_count = 148;
 
@@ -369,6 +387,15 @@ inline int gf_blocks(int64_t work, int threads) {
   if (b < 1) b = 1;
   if (b > (1LL << 30)) b = (1LL << 30);
   return (int)b;
+}
+
+inline double gf_elapsed(cudaEvent_t e0, cudaEvent_t e1) {  // seconds
+  float ms = 0.f;
+  if (cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) {
+    cudaGetLastError();
+    return 0.0;
+  }
+  return ms * 1e-3;
 }
 
 // internal entry points across translation units

@@ -1139,15 +1139,13 @@ GF_API gf_status gf_lp_apply(gf_ctx* ctx, const float* r, float* z) {
   gf_status st = gf_lp_prepare(ctx);
   if (st != GF_OK) return st;
   LpState* s = ctx->lp;
-  cudaEventRecord(ctx->ev0, ctx->stream);
+  ctx->time_begin(ctx->evs0);
   lp_forward(ctx, r, false);
   k_lp_output<float><<<gf_blocks(s->n, kLT), kLT, 0, ctx->stream>>>(s->n, s->rho, s->y, s->sc, z);
   GF_LAUNCH_CHECK(ctx, "k_lp_output");
-  cudaEventRecord(ctx->ev1, ctx->stream);
+  cudaEventRecord(ctx->evs1, ctx->stream);
   if ((st = lp_check_err(ctx)) != GF_OK) return st;   // waits for the stream
-  float ms = 0.f;
-  cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-  ctx->last_seconds = ms * 1e-3;   // device time of one application (gf_last_device_seconds)
+  ctx->time_end(ctx->evs0, ctx->evs1);
   return GF_OK;
 }
 

@@ -633,7 +633,7 @@ gf_status gf_spmv_launch(gf_ctx* ctx, int dtype, const void* x, void* y) {
   // 2-D node blocks read x in pairs (one 8- or 16-byte load per neighbour node)
   if (L.bdim == 2 && ((uintptr_t)x % (dtype == GF_F64 ? 16 : 8)) != 0)
     return gf_fail(ctx, GF_ERR_INVALID_ARG, "x must be aligned to two entries");
-  cudaEventRecord(ctx->ev0, ctx->stream);
+  ctx->time_begin(ctx->evs0);
   if (dtype == GF_F64)
     GF_ROWS_LAUNCH(ctx, ctx->stream, L, (k_spmv<Walk, double, double, double>),
                    (const double*)val, (const double*)x, (double*)y);
@@ -641,11 +641,9 @@ gf_status gf_spmv_launch(gf_ctx* ctx, int dtype, const void* x, void* y) {
     GF_ROWS_LAUNCH(ctx, ctx->stream, L, (k_spmv<Walk, float, float, float>),
                    (const float*)val, (const float*)x, (float*)y);
   GF_LAUNCH_CHECK(ctx, "k_spmv");
-  cudaEventRecord(ctx->ev1, ctx->stream);
-  GF_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
-  float ms = 0.f;
-  cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-  ctx->last_seconds = ms * 1e-3;
+  cudaEventRecord(ctx->evs1, ctx->stream);
+  GF_CUDA(ctx, cudaEventSynchronize(ctx->evs1));
+  ctx->time_end(ctx->evs0, ctx->evs1);
   return GF_OK;
 }
 
@@ -1091,7 +1089,8 @@ gf_status run_mixed(gf_ctx* ctx, const gf_solve_opts* o, int maxit, int check,
   GF_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-  info->seconds = ctx->last_seconds = ms * 1e-3;
+  info->seconds = ms * 1e-3;
+  ctx->set_seconds(info->seconds);
   info->iterations = fp32_iters + fp64_iters;
   info->fallback = fp64_fallback ? 1 : 0;
   info->outer = updates;
@@ -1358,7 +1357,8 @@ gf_status run_fcg(gf_ctx* ctx, const gf_solve_opts* o, int maxit, int check,
   GF_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-  info->seconds = ctx->last_seconds = ms * 1e-3;
+  info->seconds = ms * 1e-3;
+  ctx->set_seconds(info->seconds);
   info->iterations = hs.iter;
   info->outer = 1;
   info->fallback = fallback && learned ? 1 : 0;
@@ -1546,7 +1546,8 @@ gf_status gf_solve_run(gf_ctx* ctx, const gf_solve_opts* o, gf_solve_info* info)
     GF_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-    info->seconds = ctx->last_seconds = ms * 1e-3;
+    info->seconds = ms * 1e-3;
+    ctx->set_seconds(info->seconds);
     double* r64 = (double*)w + 7 * (size_t)n;
     double rrt = 0.0, ff = 0.0;
     if ((st = residual64(ctx, r64, &rrt)) != GF_OK) return st;
@@ -1607,7 +1608,8 @@ gf_status gf_solve_run(gf_ctx* ctx, const gf_solve_opts* o, gf_solve_info* info)
     GF_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-    info->seconds = ctx->last_seconds = ms * 1e-3;
+    info->seconds = ms * 1e-3;
+    ctx->set_seconds(info->seconds);
     info->iterations = iters;
     info->outer = 1;
     info->rel_residual = rr0 > 0.0 ? std::sqrt(rr / rr0) : 0.0;
@@ -1911,7 +1913,8 @@ extern "C" GF_API gf_status gf_dist_pcg(gf_ctx* ctx, const gf_solve_opts* o,
   GF_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-  info->seconds = ctx->last_seconds = ms * 1e-3;
+  info->seconds = ms * 1e-3;
+  ctx->set_seconds(info->seconds);
   info->iterations = iters;
   info->outer = 1;
   info->rel_residual = hs.rr0 > 0.0 ? std::sqrt(hs.rr / hs.rr0) : 0.0;  // recursive, all ranks

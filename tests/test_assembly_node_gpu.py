@@ -61,7 +61,7 @@ def fan(k):
     return xy, conn
 
 
-# Rows of 2 (2 k + 1) slots: a 2-D tile of 128 KB and less holds k = 48, not k = 56 (FP64);
+# Rows of 2 (2 k + 1) slots: a 2-D tile of 112 KB and less holds k = 48, not k = 56 (FP64);
 # FP64 only, since the slivers are beyond the FP32 tolerance.
 @pytest.mark.parametrize("k", [20, 48, 56])
 def test_wide_rows_2d(oracle, k):
@@ -89,3 +89,29 @@ def test_distorted_brick8_takes_fp64_geometry(oracle):
     xyz[:, 0] = np.where(np.abs(xyz[:, 0] - 1 / 3) < 1e-9,
                          0.02 + 0.6 * xyz[:, 1] * xyz[:, 2], xyz[:, 0])
     check(mg.BRICK8, 2, xyz, m.conn, None, TOL, [_lib.GF_SCATTER_AUTO], oracle)
+
+
+# FP64 Brick8 takes the node kernel from a node per lane of every SM's warp on (3552 nodes on 148
+# SMs): the last warp full (4032 = 144 x 28) and ragged, on both sides of the line.
+@pytest.mark.parametrize("n,ng", [((17, 15, 13), 2), ((16, 15, 14), 3), ((13, 14, 15), 2)])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_brick8_fp64_node_kernel_matches_oracle(oracle, n, ng, shuffled):
+    m = mg.structured(mg.BRICK8, n, jitter=0.1, seed=3, ngauss=ng)
+    E = mg.lognormal_iid(m, 0.5, seed=4)
+    xy, conn = m.coords, m.conn
+    if shuffled:
+        r = np.random.default_rng(1)
+        p, q = r.permutation(m.nnodes), r.permutation(m.nelem)
+        xy = np.empty_like(m.coords)
+        xy[p] = m.coords
+        conn, E = (p[m.conn - 1] + 1).astype(np.int32)[q], E[q]
+    # row by row, without dense matrices
+    from gpufem_b200.fem import Context
+    ro, co, vo = oracle.assemble(mg.BRICK8, ng, xy, conn, 210e3, 0.3, E_elem=E)
+    with Context(0) as ctx:
+        ctx.mesh_create(mg.BRICK8, xy, conn, ng, 210e3, E, 0.3, _lib.GF_PLANE_STRESS)
+        for scatter in (_lib.GF_SCATTER_OWNER, _lib.GF_SCATTER_AUTO):
+            ctx.assemble(_lib.GF_F64, scatter)
+            rn, ci, v = ctx.ell_download(_lib.GF_F64)
+            assert np.array_equal(rn, ro) and np.array_equal(ci, co)
+            assert (np.abs(v - vo).max(0) <= TOL[_lib.GF_F64] * np.abs(vo).max(0)).all()
