@@ -6,17 +6,22 @@
 // A CTA holds its slices of the matrix (node-block slices, gf_sell.cu) in shared memory for the
 // whole solve.  A slice's 32 nodes are a warp, each lane with its rows of r and p in registers;
 // where slices are few, further warps take a share of the slice's neighbours in the product.
-// The direction p lives in the CTAs' shared memory, a range of nodes to a CTA, and is gathered
-// from there.  An iteration has three cluster barriers: p.q, then (r.z, r.r), then the new p.
-// A CTA stores its part of a sum to every CTA before the barrier and each adds all parts after
-// it, in the same order everywhere, so a solve is reproducible.
+// Where a whole direction vector fits besides, every CTA keeps one and a node's owner stores its
+// new values to the CTAs that read them (a mask per node, from the columns), so that the product
+// gathers from its own shared memory; else the direction lives in the CTAs' shared memory, a
+// range of nodes to a CTA, and is gathered from there.  An iteration has three cluster barriers:
+// p.q, then (r.z, r.r), then the new p.  A CTA stores its part of a sum to every CTA before the
+// barrier and each adds all parts after it, in the same order everywhere, so a solve is
+// reproducible.
 //
-// Microseconds per iteration (FP64 Jacobi-PCG, the three-kernel loop in brackets): Q4 64 x 64
-// 3.7 (9.8), Q8 20 x 20 3.9 (9.9), Brick8 6^3 5.9 (15.4), Brick20 4^3 8.1 (22.2).  What is left is
-// latency: a cluster barrier is 0.2 us, a sum with its barrier about 0.6.  The matrix has to fit
-// the 16 CTAs' shared memory (3.4 MB with the vectors): read from L2 instead, 16 SMs took 22.6 us
-// on Q8 64 x 64, where the loop takes 10.4 on all of them, and a grid-wide version (148 CTAs,
-// sums through global memory) took 13.
+// Microseconds per iteration (FP64 Jacobi-PCG; gathering from the other CTAs; the three-kernel
+// loop): Q4 64 x 64 3.4 (3.7; 9.8), Q8 20 x 20 3.5 (4.0; 9.9), Brick8 6^3 4.4 (5.8; 15.4), Brick20
+// 4^3 5.5 (8.1; 22.2); FP32 Brick8 11^3 5.3 (9.0).  What is left is latency: a cluster barrier is
+// 0.2 us, a sum or a store to other CTAs with its barrier about 0.6.  The matrix has to fit the 16
+// CTAs' shared memory (3.4 MB with the vectors): read from L2 instead, 16 SMs took 22.6 us on Q8
+// 64 x 64, where the loop takes 10.4 on all of them, and a grid-wide version (148 CTAs, sums
+// through global memory) took 13.  Storing z before the second barrier, so that readers form p
+// themselves and the third barrier goes, cost more in gathers than the barrier (Q4 64 4.3 us).
 #include <algorithm>
 
 #include "gf_internal.cuh"
@@ -57,6 +62,7 @@ __device__ __forceinline__ void st_cluster(uint32_t a, double v) {
 __device__ __forceinline__ void st_cluster(uint32_t a, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
+// The DIM values of a node: from the cluster, from this CTA's shared memory, and to the cluster
 template <int DIM, typename V>
 __device__ __forceinline__ void ld_node(uint32_t a, V (&v)[DIM]) {
   if constexpr (DIM == 2 && sizeof(V) == 8) {
@@ -66,6 +72,33 @@ __device__ __forceinline__ void ld_node(uint32_t a, V (&v)[DIM]) {
   } else {
 #pragma unroll
     for (int c = 0; c < DIM; ++c) v[c] = ld_cluster(a + c * (uint32_t)sizeof(V), V(0));
+  }
+}
+
+template <int DIM, typename V>
+__device__ __forceinline__ void ld_node(const unsigned char* a, V (&v)[DIM]) {
+  if constexpr (DIM == 2 && sizeof(V) == 8) {
+    const double2 q = *reinterpret_cast<const double2*>(a);
+    v[0] = q.x;
+    v[1] = q.y;
+  } else if constexpr (DIM == 2) {
+    const float2 q = *reinterpret_cast<const float2*>(a);
+    v[0] = q.x;
+    v[1] = q.y;
+  } else {
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) v[c] = reinterpret_cast<const V*>(a)[c];
+  }
+}
+template <int DIM, typename V>
+__device__ __forceinline__ void st_node(uint32_t a, const V (&v)[DIM]) {
+  if constexpr (DIM == 2 && sizeof(V) == 8) {
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v[0]), "d"(v[1]) : "memory");
+  } else if constexpr (DIM == 2) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v[0]), "f"(v[1]) : "memory");
+  } else {
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) st_cluster(a + c * (uint32_t)sizeof(V), v[c]);
   }
 }
 
@@ -114,13 +147,16 @@ struct ClusterArgs {
   SolveScalars* sc;
 };
 
-// Shared memory besides the slices: sums, directions, x and 1 / diagonal, partial products.
-template <int DIM, typename V>
-__host__ __device__ constexpr size_t cluster_vectors(int S, int H) {
-  return sizeof(double) * (3 * kCluster + 64) + sizeof(V) * DIM * 32 * (size_t)S * (2 + H);
+// Shared memory besides the slices: sums, directions (COPY: all of them, and the masks), x and
+// 1 / diagonal, partial products.
+template <int DIM, typename V, bool COPY>
+__host__ __device__ constexpr size_t cluster_vectors(int S, int H, int nnodes) {
+  return sizeof(double) * (3 * kCluster + 64) + sizeof(V) * DIM * 32 * (size_t)S * (1 + H) +
+         (COPY ? (sizeof(V) * DIM * nnodes + 15) / 16 * 16 + sizeof(uint32_t) * 32 * S
+               : sizeof(V) * DIM * 32 * (size_t)S);
 }
 
-template <int DIM, typename V>
+template <int DIM, typename V, bool COPY>
 __global__ void __launch_bounds__(kThreadsMax)
 k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ dinv,
               V* __restrict__ x, V* __restrict__ r, V* __restrict__ p) {
@@ -131,8 +167,11 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
   double* partA = reinterpret_cast<double*>(smem_raw);       // [1][kCluster]
   double* partB = partA + kCluster;                          // [2][kCluster]
   double* sh = partB + 2 * kCluster;                         // [2][32]
-  V* sp = reinterpret_cast<V*>(sh + 64);                     // [per][DIM] directions of this CTA's nodes
-  V* sx = sp + (size_t)per * DIM;                            // [DIM][per] this CTA's slots
+  // directions: [per][DIM] of this CTA's nodes, or [nnodes][DIM] where copies are kept
+  V* sp = reinterpret_cast<V*>(sh + 64);
+  uint32_t* smask = reinterpret_cast<uint32_t*>(                // [per] CTAs that read a node's
+      reinterpret_cast<unsigned char*>(sp) + (sizeof(V) * DIM * A.nnodes + 15) / 16 * 16);
+  V* sx = COPY ? reinterpret_cast<V*>(smask + per) : sp + (size_t)per * DIM;  // [DIM][per] slots
   V* sd = sx + (size_t)per * DIM;                            // [DIM][per]
   V* sq = sd + (size_t)per * DIM;                            // [H - 1][DIM][per]
   V* sv = sq + (size_t)per * DIM * (H - 1);                  // the CTA's slices: values, then
@@ -147,8 +186,23 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
   auto home = [&](int b) {   // address of node b's direction
     return map_rank(sp_addr + (uint32_t)((b % per) * DIM * sizeof(V)), (uint32_t)(b / per));
   };
+  auto mask_of = [&](int b) {   // address of node b's mask
+    return map_rank((uint32_t)__cvta_generic_to_shared(smask) + (uint32_t)(b % per) * 4, (uint32_t)(b / per));
+  };
+  if constexpr (COPY) {
+    for (int i = threadIdx.x; i < per; i += blockDim.x) smask[i] = 0;
+    cluster_sync();
+  }
   for (int64_t i = threadIdx.x; i < cnt * (DIM * DIM); i += blockDim.x) sv[i] = val[o0 * (DIM * DIM) + i];
-  for (int64_t i = threadIdx.x; i < cnt; i += blockDim.x) sa[i] = home(A.col[o0 + i]);
+  for (int64_t i = threadIdx.x; i < cnt; i += blockDim.x) {
+    const int b = A.col[o0 + i];
+    if constexpr (COPY) {
+      sa[i] = (uint32_t)(b * DIM * sizeof(V));
+      asm volatile("red.shared::cluster.or.b32 [%0], %1;" ::"r"(mask_of(b)), "r"(1u << cluster_rank()) : "memory");
+    } else {
+      sa[i] = home(b);
+    }
+  }
   int w = 0;
   const V* vp = sv + lane;
   const uint32_t* ap = sa + lane;
@@ -161,7 +215,23 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
   const int li = ks * 32 + lane, slot = k0 * 32 + li;
   const bool on = h == 0 && k0 + ks < k1 && slot < A.nnodes;
   const int a = on ? A.perm[slot] : 0;
-  const uint32_t mine = home(a);
+  uint32_t mine = 0, readers = 0;
+  if constexpr (COPY) {
+    cluster_sync();   // the masks are complete
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(readers) : "r"(mask_of(a)) : "memory");
+    mine = sp_addr + (uint32_t)(a * DIM * sizeof(V));
+    if (!on) readers = 0;
+  } else {
+    mine = home(a);
+  }
+  // the lane's direction to where it is read
+  auto publish = [&](const V (&v)[DIM]) {
+    if constexpr (COPY) {
+      for (uint32_t m = readers; m; m &= m - 1) st_node<DIM, V>(map_rank(mine, __ffs(m) - 1), v);
+    } else if (on) {
+      st_node<DIM, V>(mine, v);
+    }
+  };
   V rv[DIM], pv[DIM];
 #pragma unroll
   for (int c = 0; c < DIM; ++c) {
@@ -172,8 +242,8 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
       sx[c * per + li] = on ? x[i] : V(0);
       sd[c * per + li] = on ? (A.jacobi ? dinv[i] : V(1)) : V(0);
     }
-    if (on) st_cluster(mine + c * (uint32_t)sizeof(V), pv[c]);
   }
+  publish(pv);
   double rz = sc->rzn, rr = sc->rr;
   const double tol2 = sc->tol2;
   int iter = sc->iter, done = 0;
@@ -186,7 +256,10 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
 #pragma unroll 4
     for (int s = h; s < w; s += H) {
       V g[DIM];
-      ld_node<DIM, V>(ap[32 * s], g);
+      if constexpr (COPY)
+        ld_node<DIM, V>(reinterpret_cast<const unsigned char*>(sp) + ap[32 * s], g);
+      else
+        ld_node<DIM, V>(ap[32 * s], g);
       const V* e = vp + s * (DIM * DIM * 32);
 #pragma unroll
       for (int c = 0; c < DIM; ++c)
@@ -234,10 +307,8 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
     if (rr <= tol2) done = 1;
     else if (iter >= maxit) done = 3;
 #pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      pv[c] = fma(beta, pv[c], zv[c]);
-      if (on) st_cluster(mine + c * (uint32_t)sizeof(V), pv[c]);
-    }
+    for (int c = 0; c < DIM; ++c) pv[c] = fma(beta, pv[c], zv[c]);
+    publish(pv);
     cluster_sync();
   }
   cluster_sync();   // no CTA leaves while another may still write to it
@@ -257,8 +328,8 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
   }
 }
 
-template <int DIM, typename V>
-gf_status run_cluster(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V* p, int iters, int* ran) {
+template <int DIM, typename V, bool COPY>
+gf_status run_cluster_as(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V* p, int iters, int* ran) {
   *ran = 0;
   const int nslice = (ctx->nnodes + 31) / 32;
   const int S = (nslice + kCluster - 1) / kCluster;
@@ -266,10 +337,10 @@ gf_status run_cluster(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V* p
   // a CTA's slices at the widest row
   const size_t slices = (size_t)S * 32 * (ctx->W / DIM) * (DIM * DIM * sizeof(V) + 4);
   int H = 1;
-  while (S * H * 2 <= 16 && cluster_vectors<DIM, V>(S, H * 2) + slices <= kSmemMax) H *= 2;
-  const size_t sm = cluster_vectors<DIM, V>(S, H) + slices;
+  while (S * H * 2 <= 16 && cluster_vectors<DIM, V, COPY>(S, H * 2, ctx->nnodes) + slices <= kSmemMax) H *= 2;
+  const size_t sm = cluster_vectors<DIM, V, COPY>(S, H, ctx->nnodes) + slices;
   if (sm > kSmemMax) return GF_OK;
-  auto kern = k_pcg_cluster<DIM, V>;
+  auto kern = k_pcg_cluster<DIM, V, COPY>;
   GF_CUDA(ctx, gf_smem_attr(kern, sm));
   GF_CUDA(ctx, gf_func_attr((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   ClusterArgs A{ctx->nnodes, S, H, iters, dinv != nullptr, ctx->d_sell_perm, ctx->d_sell_w,
@@ -295,6 +366,14 @@ gf_status run_cluster(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V* p
   GF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   *ran = 1;
   return GF_OK;
+}
+
+// With copies of the direction where they fit.
+template <int DIM, typename V>
+gf_status run_cluster(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V* p, int iters, int* ran) {
+  const gf_status st = run_cluster_as<DIM, V, true>(ctx, val, dinv, x, r, p, iters, ran);
+  if (st != GF_OK || *ran) return st;
+  return run_cluster_as<DIM, V, false>(ctx, val, dinv, x, r, p, iters, ran);
 }
 
 }  // namespace

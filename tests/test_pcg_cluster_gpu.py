@@ -92,3 +92,40 @@ def test_solves_repeat_bit_for_bit():
             ctx.solve(_lib.GF_SOLVER_PCG, _lib.GF_F64, tol=1e-10, max_iter=20000)
             u.append(ctx.solution())
         assert np.array_equal(*u)
+
+
+# Copies of the direction in every CTA and directions gathered from their homes, on both sides of
+# the sizes where the copies stop fitting (5,041 and 5,776 nodes in 2-D, 1,000 and 1,331 in 3-D);
+# shuffled node ids give a node up to 16 CTAs that read it.
+@pytest.mark.parametrize("et,n", [(mg.Q4, (70, 70)), (mg.Q4, (75, 75)), (mg.Q8, (20, 17)),
+                                  (mg.BRICK8, (9, 9, 9)), (mg.BRICK8, (10, 10, 10)),
+                                  (mg.BRICK20, (4, 3, 3))])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_copies_and_gathers_match_numpy(et, n, shuffled):
+    from gpufem_b200.fem import Context
+    m = mg.clamp_and_load(mg.structured(et, n, jitter=0.05, seed=2, ngauss=2))
+    m.E = mg.lognormal_iid(m, 0.5, seed=3)
+    xy, conn, sup, f = m.coords, m.conn, m.supports, m.f
+    if shuffled:
+        q = np.random.default_rng(1).permutation(m.nnodes)
+        xy, f = np.empty_like(m.coords), np.empty_like(m.f)
+        xy[q] = m.coords
+        f.reshape(-1, m.dim)[q] = m.f.reshape(-1, m.dim)
+        conn = (q[m.conn - 1] + 1).astype(np.int32)
+        sup = m.supports.copy()
+        sup[:, 0] = q[m.supports[:, 0].astype(int) - 1] + 1
+    with Context(0) as ctx:
+        ctx.mesh_create(m.elem_type, xy, conn, m.ngauss, m.E0, m.E, m.nu)
+        ctx.set_supports(sup)
+        ctx.set_force(f)
+        ctx.assemble(_lib.GF_F64, _lib.GF_SCATTER_AUTO)
+        ctx.apply_constraints(_lib.GF_BC_ELIMINATION)
+        rn, ci, v = ctx.ell_download(_lib.GF_F64)
+        mask = np.arange(ci.shape[0])[:, None] < rn[None, :]
+        rows = np.broadcast_to(np.arange(rn.size)[None, :], ci.shape)
+        K = sp.csr_matrix((v[mask], (rows[mask], ci[mask])), shape=(rn.size, rn.size))
+        b = ctx.get_force()
+        for its in (1, 4):
+            ctx.solve(_lib.GF_SOLVER_PCG, _lib.GF_F64, tol=1e-30, max_iter=its, raise_on_error=False)
+            want = pcg(K, b, 1.0 / K.diagonal(), its)
+            assert np.linalg.norm(ctx.solution() - want) <= 1e-10 * np.linalg.norm(want)
