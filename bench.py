@@ -703,8 +703,9 @@ def run_gpu_arm(args):
             dist.barrier()
         torch.cuda.synchronize()
 
-    # "auto" resolves as the library's GF_SCATTER_AUTO does: atomic in 3-D, owner in 2-D
-    sname = args.scatter if args.scatter != "auto" else ("atomic" if m.dim == 3 else "owner")
+    # "auto" resolves as the library's GF_SCATTER_AUTO does on these workloads
+    sname = args.scatter if args.scatter != "auto" else (
+        "atomic" if m.nen == 20 else "owner")
     scatter = {"owner": _lib.GF_SCATTER_OWNER, "colour": _lib.GF_SCATTER_COLOR,
                "atomic": _lib.GF_SCATTER_ATOMIC}[sname]
     for _ in range(args.warmup):
@@ -776,24 +777,26 @@ def run_gpu_arm(args):
     hbm, peak_kind = peaks()
     alg_bytes = nnz * esize + m.nnodes * m.dim * esize + m.nelem * (m.nen * 4 + esize)
     achieved = alg_bytes / per_step / 1e9
-    # dominant kernel (owner schedule: k_assemble_owner_node for 2-D FP32, else
+    # dominant kernel (owner schedule: k_node_rows_2d, k_node_rows_b8, for Brick20
     # k_assemble_owner): K values written once, plus what it must read — J^-1 and w*detJ
-    # per element and Gauss point (the 2-D FP32 kernel reads w*detJ*E, the modulus folded
-    # in; the other reads the moduli apart), and per incidence the element id, local node
+    # per element and Gauss point (the node kernels read w*detJ*E, the modulus folded in;
+    # the other reads the moduli apart), and per incidence the element id, local node
     # index and nen neighbour slots
     ngp = m.ngauss ** m.dim
     t_geo = float(np.mean([a for a, _ in split]))
     t_dom = float(np.mean([b for _, b in split]))
     if sname == "owner":
         ninc = m.nelem * m.nen
-        node_kernel = m.dim == 2 and esize == 4
+        node_kernel = m.nen != 20
         dom_bytes = (nnz * esize + m.nelem * ngp * (m.dim * m.dim + 1) * esize
                      + (0 if node_kernel else m.nelem * esize)
                      + ninc * (4 + 1 + 2 * m.nen) + (m.nnodes + 1) * 4)
-        dom_name = "k_assemble_owner_node" if node_kernel else "k_assemble_owner"
+        dom_name = ("k_assemble_owner" if not node_kernel else
+                    "k_node_rows_2d" if m.dim == 2 else "k_node_rows_b8")
     else:
         dom_bytes = alg_bytes
         dom_name = ("k_assemble (all colour passes)" if sname == "colour" else
+                    "k_assemble_b20" if m.nen == 20 else
                     "k_assemble (atomic)") + " + K zero-fill"
     traffic = traffic_asm = None
     tfile = ROOT / "profiles" / "ncu_traffic.json"
@@ -925,7 +928,7 @@ def run_gpu_arm(args):
             "roofline_assembly": {"bound": "hbm", "achieved": achieved, "peak": hbm,
                                   "unit": "GB/s", "frac": achieved / hbm,
                                   "traffic": traffic_asm, "algorithmic_bytes": alg_bytes,
-                                  "kernels_us": {"k_elem_geometry": t_geo * 1e6,
+                                  "kernels_us": {"k_geometry": t_geo * 1e6,
                                                  dom_name: t_dom * 1e6}},
             "roofline_spmv": {"bound": "hbm", "achieved": spmv_bytes / t_spmv / 1e9, "peak": hbm,
                               "unit": "GB/s", "frac": spmv_bytes / t_spmv / 1e9 / hbm,

@@ -539,7 +539,8 @@ GF_API gf_status gf_assemble(gf_ctx* ctx, int32_t dtype, int32_t scatter, int32_
   // FP64 sums, 42 us at 8^3 and 48 at 21^3 against 27 and 46 with atomics (22^3: 48 and 57)
   const bool b8_small = ctx->elem_type == GF_BRICK8 && dtype == GF_F64 &&
                         ctx->nnodes <= 76 * (int64_t)ctx->sm_count;
-  if (scatter == GF_SCATTER_AUTO)
+  const bool automatic = scatter == GF_SCATTER_AUTO;
+  if (automatic)
     scatter = ctx->dim == 2 || engine == GF_ENGINE_TF32_MMA ||
                       (gf_assemble_node_fits(ctx, dtype) && !b8_small)
                   ? GF_SCATTER_OWNER
@@ -547,7 +548,12 @@ GF_API gf_status gf_assemble(gf_ctx* ctx, int32_t dtype, int32_t scatter, int32_
   if (scatter == GF_SCATTER_COLOR && ctx->ncolors == 0 &&
       (st = gf_color_build(ctx, nullptr)) != GF_OK)
     return st;
-  return gf_assemble_launch(ctx, dtype, scatter, engine);
+  st = gf_assemble_launch(ctx, dtype, scatter, engine);
+  // no room for Brick8's geometry (320 bytes an element in FP32): atomics do without
+  if (st == GF_ERR_OOM && automatic && scatter == GF_SCATTER_OWNER &&
+      ctx->elem_type == GF_BRICK8 && engine != GF_ENGINE_TF32_MMA)
+    st = gf_assemble_launch(ctx, dtype, GF_SCATTER_ATOMIC, engine);
+  return st;
 }
 
 GF_API gf_status gf_ell_convert_f64_to_f32(gf_ctx* ctx) {

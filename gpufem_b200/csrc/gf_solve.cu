@@ -13,7 +13,8 @@
 //   K3  beta; p = z + beta p; convergence flag
 // with the scalars in device memory.  Chunks of iterations are captured once
 // into a CUDA graph; the host reads the convergence flag after each chunk, and
-// kernels of a finished solve return immediately.
+// kernels of a finished solve return immediately.  Small systems run every iteration in one
+// kernel (gf_pcg_cluster.cu).
 #include <chrono>
 #include <cmath>
 #include <algorithm>
