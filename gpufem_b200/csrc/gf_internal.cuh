@@ -413,9 +413,9 @@ gf_status gf_solve_run(gf_ctx* ctx, const gf_solve_opts* o, gf_solve_info* info)
 void gf_solver_free(gf_ctx* ctx);
 // (P)CG in one kernel (gf_pcg_cluster.cu)
 gf_status gf_pcg_cluster(gf_ctx* ctx, const double* val, const double* dinv, double* x, double* r,
-                         double* p, int iters, int* ran);
+                         double* p, double eps, int iters, int* ran);
 gf_status gf_pcg_cluster(gf_ctx* ctx, const float* val, const float* dinv, float* x, float* r,
-                         float* p, int iters, int* ran);
+                         float* p, double eps, int iters, int* ran);
 void gf_dist_free(gf_ctx* ctx);
 void gf_mesh_free(gf_ctx* ctx);
 void gf_pattern_free(gf_ctx* ctx);

@@ -9,19 +9,22 @@
 // Where a whole direction vector fits besides, every CTA keeps one and a node's owner stores its
 // new values to the CTAs that read them (a mask per node, from the columns), so that the product
 // gathers from its own shared memory; else the direction lives in the CTAs' shared memory, a
-// range of nodes to a CTA, and is gathered from there.  An iteration has three cluster barriers:
-// p.q, then (r.z, r.r), then the new p.  A CTA stores its part of a sum to every CTA before the
-// barrier and each adds all parts after it, in the same order everywhere, so a solve is
+// range of nodes to a CTA, and is gathered from there.  An iteration exchanges three things: p.q,
+// then (r.z, r.r), then the new p.  With copies they are asynchronous stores that complete on a
+// barrier of the CTA they go to, which waits for their bytes alone; a buffer is written again only
+// after an answer that its reader sends when it is done with it.  Waits are bounded; a CTA that
+// gives up leaves the iteration as a whole, and the others follow.  Without copies there is a
+// cluster barrier after each.  Each CTA adds all parts of a sum in the same order, so a solve is
 // reproducible.
 //
-// Microseconds per iteration (FP64 Jacobi-PCG; gathering from the other CTAs; the three-kernel
-// loop): Q4 64 x 64 3.4 (3.7; 9.8), Q8 20 x 20 3.5 (4.0; 9.9), Brick8 6^3 4.4 (5.8; 15.4), Brick20
-// 4^3 5.5 (8.1; 22.2); FP32 Brick8 11^3 5.3 (9.0).  What is left is latency: a cluster barrier is
-// 0.2 us, a sum or a store to other CTAs with its barrier about 0.6.  The matrix has to fit the 16
-// CTAs' shared memory (3.4 MB with the vectors): read from L2 instead, 16 SMs took 22.6 us on Q8
-// 64 x 64, where the loop takes 10.4 on all of them, and a grid-wide version (148 CTAs, sums
-// through global memory) took 13.  Storing z before the second barrier, so that readers form p
-// themselves and the third barrier goes, cost more in gathers than the barrier (Q4 64 4.3 us).
+// Microseconds per iteration (FP64 Jacobi-PCG; the same with cluster barriers; gathering from the
+// other CTAs; the three-kernel loop): Q4 64 x 64 3.0 (3.4; 3.7; 9.8), Q8 20 x 20 3.1 (3.5; 4.0;
+// 9.9), Brick8 6^3 4.0 (4.4; 5.8; 15.4), Brick20 4^3 5.2 (5.5; 8.1; 22.2); FP32 Brick8 11^3 5.1
+// (5.3; 9.0).  What is left is latency: sums over a warp, a CTA and the cluster, twice.  The matrix
+// has to fit the 16 CTAs' shared memory (3.4 MB with the vectors): read from L2 instead, 16 SMs
+// took 22.6 us on Q8 64 x 64, where the loop takes 10.4 on all of them, and a grid-wide version
+// (148 CTAs, sums through global memory) took 13.  Storing z with r.z, so that readers form p
+// themselves, cost more in gathers from other CTAs than the barrier it saved (Q4 64 4.3 us).
 #include <algorithm>
 
 #include "gf_internal.cuh"
@@ -102,16 +105,69 @@ __device__ __forceinline__ void st_node(uint32_t a, const V (&v)[DIM]) {
   }
 }
 
+// Stores that complete on a barrier in the shared memory of the CTA they go to (their bytes count
+// towards its transaction count)
+__device__ __forceinline__ void st_async(uint32_t a, double v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(a),
+               "l"(__double_as_longlong(v)), "r"(bar)
+               : "memory");
+}
+template <int DIM>
+__device__ __forceinline__ void st_async_node(uint32_t a, const double (&v)[DIM], uint32_t bar) {
+  if constexpr (DIM == 2)
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(a),
+                 "l"(__double_as_longlong(v[0])), "l"(__double_as_longlong(v[1])), "r"(bar)
+                 : "memory");
+  else
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) st_async(a + 8 * c, v[c], bar);
+}
+template <int DIM>
+__device__ __forceinline__ void st_async_node(uint32_t a, const float (&v)[DIM], uint32_t bar) {
+  if constexpr (DIM == 2)
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(a),
+                 "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(bar)
+                 : "memory");
+  else
+#pragma unroll
+    for (int c = 0; c < DIM; ++c)
+      asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(a + 4 * c),
+                   "r"(__float_as_uint(v[c])), "r"(bar)
+                   : "memory");
+}
+// One thread per phase: the bytes that the phase waits for
+__device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Waits for the phase of parity `parity`; false if it does not come.
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
+  for (int k = 0; k < 20000; ++k) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(parity)
+                 : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-// Sums N values (of the first S warps) over the cluster; `part` is this CTA's [N][kCluster].
-template <int N>
-__device__ __forceinline__ void cluster_sum(double (&v)[N], int S, double* sh, double* part,
-                                            uint32_t part_addr) {
+// Sums N values (of the first S warps) over the cluster; `part` is this CTA's [N][kCluster].  The
+// CTA's parts are sent to every CTA and are awaited there: on `bar` (ASYNC), else by a cluster
+// barrier.  late: a wait of this thread has run out.  True, the same for the whole CTA, if one of
+// its threads came late; nothing was sent then.
+template <int N, bool ASYNC>
+__device__ __forceinline__ bool cluster_sum(double (&v)[N], int S, double* sh, double* part,
+                                            uint32_t part_addr, uint32_t bar, uint32_t parity,
+                                            bool& late) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < S) {
 #pragma unroll
@@ -120,15 +176,29 @@ __device__ __forceinline__ void cluster_sum(double (&v)[N], int S, double* sh, d
       if (lane == 0) sh[k * 32 + warp] = s;
     }
   }
-  __syncthreads();
+  if constexpr (ASYNC) {
+    if (__syncthreads_or(late)) return true;
+  } else {
+    __syncthreads();
+  }
   if (warp == 0) {
+    if (ASYNC && lane == 0) bar_expect(bar, N * kCluster * 8);
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       const double s = warp_sum(lane < S ? sh[k * 32 + lane] : 0.0);
-      if (lane < kCluster) st_cluster(map_rank(part_addr + (k * kCluster + cluster_rank()) * 8, lane), s);
+      const uint32_t mine = part_addr + (k * kCluster + cluster_rank()) * 8;
+      if (lane < kCluster) {
+        if constexpr (ASYNC)
+          st_async(map_rank(mine, lane), s, map_rank(bar, lane));
+        else
+          st_cluster(map_rank(mine, lane), s);
+      }
     }
   }
-  cluster_sync();
+  if constexpr (ASYNC)
+    late = !bar_wait(bar, parity);
+  else
+    cluster_sync();
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     double s = part[k * kCluster + (lane & (kCluster - 1))];
@@ -136,10 +206,12 @@ __device__ __forceinline__ void cluster_sum(double (&v)[N], int S, double* sh, d
     for (int o = kCluster / 2; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     v[k] = s;
   }
+  return false;
 }
 
 struct ClusterArgs {
   int nnodes, S, H, iters, jacobi;   // S slices per CTA, H warps per slice
+  double eps;
   const int32_t* __restrict__ perm;
   const int32_t* __restrict__ width;
   const int64_t* __restrict__ off;
@@ -151,7 +223,7 @@ struct ClusterArgs {
 // 1 / diagonal, partial products.
 template <int DIM, typename V, bool COPY>
 __host__ __device__ constexpr size_t cluster_vectors(int S, int H, int nnodes) {
-  return sizeof(double) * (3 * kCluster + 64) + sizeof(V) * DIM * 32 * (size_t)S * (1 + H) +
+  return sizeof(double) * (3 * kCluster + 64 + 4) + sizeof(V) * DIM * 32 * (size_t)S * (1 + H) +
          (COPY ? (sizeof(V) * DIM * nnodes + 15) / 16 * 16 + sizeof(uint32_t) * 32 * S
                : sizeof(V) * DIM * 32 * (size_t)S);
 }
@@ -168,7 +240,9 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
   double* partB = partA + kCluster;                          // [2][kCluster]
   double* sh = partB + 2 * kCluster;                         // [2][32]
   // directions: [per][DIM] of this CTA's nodes, or [nnodes][DIM] where copies are kept
-  V* sp = reinterpret_cast<V*>(sh + 64);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sh + 64);     // p.q; r.z and r.r; directions
+  uint32_t* count = reinterpret_cast<uint32_t*>(bars + 3);   // nodes whose directions come here
+  V* sp = reinterpret_cast<V*>(bars + 4);
   uint32_t* smask = reinterpret_cast<uint32_t*>(                // [per] CTAs that read a node's
       reinterpret_cast<unsigned char*>(sp) + (sizeof(V) * DIM * A.nnodes + 15) / 16 * 16);
   V* sx = COPY ? reinterpret_cast<V*>(smask + per) : sp + (size_t)per * DIM;  // [DIM][per] slots
@@ -189,8 +263,16 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
   auto mask_of = [&](int b) {   // address of node b's mask
     return map_rank((uint32_t)__cvta_generic_to_shared(smask) + (uint32_t)(b % per) * 4, (uint32_t)(b / per));
   };
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(bars);
   if constexpr (COPY) {
     for (int i = threadIdx.x; i < per; i += blockDim.x) smask[i] = 0;
+    if (threadIdx.x == 0) {
+      *count = 0;
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8 * k) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
     cluster_sync();
   }
   for (int64_t i = threadIdx.x; i < cnt * (DIM * DIM); i += blockDim.x) sv[i] = val[o0 * (DIM * DIM) + i];
@@ -218,6 +300,9 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
   uint32_t mine = 0, readers = 0;
   if constexpr (COPY) {
     cluster_sync();   // the masks are complete
+    for (int i = threadIdx.x; i < per; i += blockDim.x)
+      for (uint32_t m = smask[i]; m; m &= m - 1)
+        asm volatile("red.shared::cluster.add.u32 [%0], 1;" ::"r"(map_rank(bar + 24, __ffs(m) - 1)) : "memory");
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(readers) : "r"(mask_of(a)) : "memory");
     mine = sp_addr + (uint32_t)(a * DIM * sizeof(V));
     if (!on) readers = 0;
@@ -227,7 +312,10 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
   // the lane's direction to where it is read
   auto publish = [&](const V (&v)[DIM]) {
     if constexpr (COPY) {
-      for (uint32_t m = readers; m; m &= m - 1) st_node<DIM, V>(map_rank(mine, __ffs(m) - 1), v);
+      for (uint32_t m = readers; m; m &= m - 1) {
+        const uint32_t to = __ffs(m) - 1;
+        st_async_node<DIM>(map_rank(mine, to), v, map_rank(bar + 16, to));
+      }
     } else if (on) {
       st_node<DIM, V>(mine, v);
     }
@@ -243,13 +331,33 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
       sd[c * per + li] = on ? (A.jacobi ? dinv[i] : V(1)) : V(0);
     }
   }
+  if (COPY) cluster_sync();   // the counts are complete
+  const uint32_t bytes = COPY ? *count * (uint32_t)(DIM * sizeof(V)) : 0;
+  if (COPY && threadIdx.x == 0) bar_expect(bar + 16, bytes);
   publish(pv);
-  double rz = sc->rzn, rr = sc->rr;
-  const double tol2 = sc->tol2;
+  bool late = false;
+  double rz = sc->rzn, rr = sc->rr, tol2 = sc->tol2;
   int iter = sc->iter, done = 0;
+  const bool fresh = iter == 0;
+  if (fresh) {   // p = z: the first sums again, in this kernel's fixed order
+    double two[2] = {0.0, 0.0};
+    if (h == 0)
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        two[0] += (double)rv[c] * (double)pv[c];
+        two[1] += (double)rv[c] * (double)rv[c];
+      }
+    cluster_sum<2, false>(two, S, sh, partB, pb, 0, 0, late);
+    rz = two[0];
+    rr = two[1];
+    tol2 = A.eps * A.eps * rr;
+  }
+  const double rr0 = rr;
   const int maxit = sc->maxit;
-  cluster_sync();
-  for (int step = 0; step < A.iters && !done; ++step) {
+  if (!COPY) cluster_sync();
+  for (int step = 0; step < A.iters; ++step) {
+    const uint32_t parity = step & 1;
+    if (COPY) late = !bar_wait(bar + 16, parity);
     V q[DIM];
 #pragma unroll
     for (int c = 0; c < DIM; ++c) q[c] = V(0);
@@ -279,19 +387,19 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
     double sum[1] = {0.0};
 #pragma unroll
     for (int c = 0; c < DIM; ++c) sum[0] += (double)pv[c] * (double)q[c];
-    cluster_sum<1>(sum, S, sh, partA, pa);
-    const double pq = sum[0];
-    if (!(pq > 0.0) || !isfinite(pq)) {
-      done = 2;
+    if (cluster_sum<1, COPY>(sum, S, sh, partA, pa, bar, parity, late)) {
+      done = 4;
       break;
     }
+    const double pq = sum[0];
+    const bool valid = pq > 0.0 && isfinite(pq);
     const V alpha = (V)(rz / pq);
     double two[2] = {0.0, 0.0};
     V zv[DIM];
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
       zv[c] = V(0);
-      if (h == 0) {
+      if (h == 0 && valid) {
         sx[c * per + li] = fma(alpha, pv[c], sx[c * per + li]);
         rv[c] = fma(-alpha, q[c], rv[c]);
         zv[c] = rv[c] * sd[c * per + li];
@@ -299,7 +407,18 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
         two[1] += (double)rv[c] * (double)rv[c];
       }
     }
-    cluster_sum<2>(two, S, sh, partB, pb);
+    if (cluster_sum<2, COPY>(two, S, sh, partB, pb, bar + 8, parity, late)) {
+      done = 4;
+      break;
+    }
+    if (!valid) {   // the same everywhere: who came late to p.q has left above
+      done = 2;
+      break;
+    }
+    if (COPY && __syncthreads_or(late)) {
+      done = 4;
+      break;
+    }
     const V beta = (V)(two[0] / rz);
     rz = two[0];
     rr = two[1];
@@ -308,9 +427,13 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
     else if (iter >= maxit) done = 3;
 #pragma unroll
     for (int c = 0; c < DIM; ++c) pv[c] = fma(beta, pv[c], zv[c]);
+    if (done || step + 1 == A.iters) break;   // nobody reads the next directions
+    if (COPY && threadIdx.x == 0) bar_expect(bar + 16, bytes);
     publish(pv);
-    cluster_sync();
+    if (!COPY) cluster_sync();
   }
+  if (done == 4)
+    for (int k = 0; k < 100; ++k) __nanosleep(1000);   // what is under way arrives
   cluster_sync();   // no CTA leaves while another may still write to it
   if (on)
 #pragma unroll
@@ -321,6 +444,10 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
       p[i] = pv[c];
     }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (fresh) {
+      sc->rr0 = rr0;
+      sc->tol2 = tol2;
+    }
     sc->rzn = rz;
     sc->rr = rr;
     sc->iter = iter;
@@ -329,8 +456,10 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
 }
 
 template <int DIM, typename V, bool COPY>
-gf_status run_cluster_as(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V* p, int iters, int* ran) {
+gf_status run_cluster_as(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V* p, double eps,
+                         int iters, int* ran) {
   *ran = 0;
+  if (iters < 1) return GF_OK;
   const int nslice = (ctx->nnodes + 31) / 32;
   const int S = (nslice + kCluster - 1) / kCluster;
   if (S > kThreadsMax / 32) return GF_OK;
@@ -343,7 +472,7 @@ gf_status run_cluster_as(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V
   auto kern = k_pcg_cluster<DIM, V, COPY>;
   GF_CUDA(ctx, gf_smem_attr(kern, sm));
   GF_CUDA(ctx, gf_func_attr((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  ClusterArgs A{ctx->nnodes, S, H, iters, dinv != nullptr, ctx->d_sell_perm, ctx->d_sell_w,
+  ClusterArgs A{ctx->nnodes, S, H, iters, dinv != nullptr, eps, ctx->d_sell_perm, ctx->d_sell_w,
                 ctx->d_sell_off, ctx->d_sell_col, ctx->d_scal};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -364,34 +493,38 @@ gf_status run_cluster_as(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V
   GF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, ctx->d_scal, sizeof(SolveScalars), cudaMemcpyDeviceToHost,
                                ctx->stream));
   GF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  if (static_cast<const SolveScalars*>(ctx->h_pinned)->done == 4)
+    return gf_fail(ctx, GF_ERR_CUDA, "PCG on a cluster: a wait for another CTA timed out");
   *ran = 1;
   return GF_OK;
 }
 
 // With copies of the direction where they fit.
 template <int DIM, typename V>
-gf_status run_cluster(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V* p, int iters, int* ran) {
-  const gf_status st = run_cluster_as<DIM, V, true>(ctx, val, dinv, x, r, p, iters, ran);
+gf_status run_cluster(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V* p, double eps, int iters,
+                      int* ran) {
+  const gf_status st = run_cluster_as<DIM, V, true>(ctx, val, dinv, x, r, p, eps, iters, ran);
   if (st != GF_OK || *ran) return st;
-  return run_cluster_as<DIM, V, false>(ctx, val, dinv, x, r, p, iters, ran);
+  return run_cluster_as<DIM, V, false>(ctx, val, dinv, x, r, p, eps, iters, ran);
 }
 
 }  // namespace
 
-// Runs up to `iters` iterations of the (P)CG whose state is in x, r, p and the context's scalars
+// Runs up to `iters` iterations of the (P)CG to the tolerance eps whose state is in x, r, p and the
+// context's scalars
 // (iter, rr, rzn, done updated and read back to the pinned copy).  *ran = 0: the system is not
 // one for this kernel, and nothing was done.  dinv = null: no preconditioner.
 gf_status gf_pcg_cluster(gf_ctx* ctx, const double* val, const double* dinv, double* x, double* r,
-                         double* p, int iters, int* ran) {
+                         double* p, double eps, int iters, int* ran) {
   *ran = 0;
-  if (ctx->sell_bdim == 2) return run_cluster<2, double>(ctx, val, dinv, x, r, p, iters, ran);
-  if (ctx->sell_bdim == 3) return run_cluster<3, double>(ctx, val, dinv, x, r, p, iters, ran);
+  if (ctx->sell_bdim == 2) return run_cluster<2, double>(ctx, val, dinv, x, r, p, eps, iters, ran);
+  if (ctx->sell_bdim == 3) return run_cluster<3, double>(ctx, val, dinv, x, r, p, eps, iters, ran);
   return GF_OK;
 }
 gf_status gf_pcg_cluster(gf_ctx* ctx, const float* val, const float* dinv, float* x, float* r,
-                         float* p, int iters, int* ran) {
+                         float* p, double eps, int iters, int* ran) {
   *ran = 0;
-  if (ctx->sell_bdim == 2) return run_cluster<2, float>(ctx, val, dinv, x, r, p, iters, ran);
-  if (ctx->sell_bdim == 3) return run_cluster<3, float>(ctx, val, dinv, x, r, p, iters, ran);
+  if (ctx->sell_bdim == 2) return run_cluster<2, float>(ctx, val, dinv, x, r, p, eps, iters, ran);
+  if (ctx->sell_bdim == 3) return run_cluster<3, float>(ctx, val, dinv, x, r, p, eps, iters, ran);
   return GF_OK;
 }

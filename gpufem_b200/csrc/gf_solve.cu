@@ -734,7 +734,8 @@ gf_status run_cg(gf_ctx* ctx, MatLayout L, const TK* val, const V* b, CgVecs vv,
   // iterations)
   for (;;) {
     int ran = 0;
-    gf_status st = gf_pcg_cluster(ctx, val, dinv, x, r, p, max_seconds > 0.0 ? check_every : maxit, &ran);
+    gf_status st = gf_pcg_cluster(ctx, val, dinv, x, r, p, eps,
+                                  max_seconds > 0.0 ? check_every : maxit, &ran);
     if (st != GF_OK) return st;
     if (!ran) break;
     if (!hs->done && max_seconds > 0.0 &&
