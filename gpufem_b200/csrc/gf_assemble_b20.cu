@@ -10,12 +10,13 @@
 // lanes (element, row): the rows of neighbouring elements' nodes lie 12 or 24 bytes apart in
 // a column of the ELL, so the lanes share lines.  Now L2 takes 140-150 G sectors of reductions
 // a second that miss it (1300 sectors per FP32 element; DRAM reads and writes K once), whatever
-// the order of the elements; from 52^3 (FP32) that is all that is left of the time.
+// the order of the elements; from 52^3 (FP32) that is all that is left of the time, and the
+// lines are fetched to L2 ahead of the reductions.
 //   us, against a thread per node pair:    FP32  FP64
 //   Brick20   8^3                    32 -> 26   35 -> 30
 //   Brick20  24^3                  191 -> 160  375 -> 277
 //   Brick20  48^3                1353 -> 1060  2770 -> 2490
-//   Brick20  64^3                3159 -> 3104  6519 -> 6433
+//   Brick20  64^3                3159 -> 2959  6519 -> 6433
 // A warp per element, so that only the reductions need the whole CTA; eight elements (four in
 // FP64) fill 24 lanes of a reduction and two CTAs an SM.  CTAs start the reductions at
 // different nodes (FP64 48^3 2474 -> 2171 us when its K was resident, nothing else).
@@ -178,7 +179,7 @@ __global__ void __launch_bounds__(B20<T, NG1>::THREADS, 2)
 k_assemble_b20(int nelem, int n, const int32_t* __restrict__ conn,
                const double* __restrict__ coords, const T* __restrict__ Eel,
                const int32_t* __restrict__ einc, const uint16_t* __restrict__ inc_slot,
-               const AsmTables* __restrict__ tab, T lam1, T mu1, T* __restrict__ K) {
+               const AsmTables* __restrict__ tab, T lam1, T mu1, bool ahead, T* __restrict__ K) {
   using L = B20<T, NG1>;
   constexpr int NGP = L::NGP, E = L::E, SS = L::SS, N = L::N, kBT = L::THREADS;
   constexpr bool f64 = sizeof(T) == 8;
@@ -251,6 +252,23 @@ k_assemble_b20(int nelem, int n, const int32_t* __restrict__ conn,
     buf ^= 1;
     fetch_data(grp + gridDim.x, ring, buf);
     fetch_ids(grp + 2 * gridDim.x, ring == 2 ? 0 : ring + 1);
+    if (ahead) {
+      // the lines that this group's reductions touch, to L2 during the products: lanes
+      // (pair, element), one prefetch where neighbouring elements share a line
+      const int e = lane % E, last = ne - 1;
+      for (int pr = warp * (32 / E) + lane / E; pr < SS; pr += kBT / 32 * (32 / E)) {
+        const T* q = K + (int64_t)snode[min(e, last) * NEN + pr / NEN] * DIM +
+                     (int64_t)sslot[min(e, last) * SS + pr] * n3;
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+          const uint64_t line = (uint64_t)(q + b * (int64_t)n) / 128;
+          const uint64_t end = ((uint64_t)(q + b * (int64_t)n + 3) - 1) / 128;
+          const uint64_t left = __shfl_up_sync(0xffffffffu, line, 1);
+          if (e == 0 || line != left) asm volatile("prefetch.global.L2 [%0];" ::"l"(line * 128));
+          if (e == E - 1 && end != line) asm volatile("prefetch.global.L2 [%0];" ::"l"(end * 128));
+        }
+      }
+    }
     if (warp < ne) {
       T* G = sG + warp * GS;
       T* X = sX + warp * NEN * 4;
@@ -393,9 +411,13 @@ gf_status launch_b20(gf_ctx* ctx, const AsmTables* d_tab, T* K) {
   GF_CUDA(ctx, gf_smem_attr(kern, L::bytes));
   const T* Eel = sizeof(T) == 8 ? (const T*)ctx->d_Eel : (const T*)ctx->d_Eel32;
   const int groups = (ctx->nelem + L::E - 1) / L::E;
+  // from 1.5 GB of K on, reductions find their lines slower than L2 takes them (FP32 52^3 1605 ->
+  // 1499 us with the lines fetched ahead, 64^3 3247 -> 2959, FP64 44^3 1930 -> 1831); below, the
+  // extra requests cost (FP32 48^3 1032 -> 1176; FP64 36^3 900 -> 896)
+  const bool ahead = (int64_t)ctx->n * ctx->W * (int64_t)sizeof(T) > 1500000000;
   kern<<<std::min(groups, ctx->sm_count * 2), L::THREADS, L::bytes, ctx->stream>>>(
       ctx->nelem, ctx->n, ctx->d_conn, ctx->d_coords64, Eel, ctx->d_einc, ctx->d_inc_slot, d_tab,
-      T(ctx->lam1), T(ctx->mu1), K);
+      T(ctx->lam1), T(ctx->mu1), ahead, K);
   GF_LAUNCH_CHECK(ctx, "k_assemble_b20");
   return GF_OK;
 }

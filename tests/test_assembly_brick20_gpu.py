@@ -53,3 +53,25 @@ def test_more_groups_than_ctas(dtype):
     scale = np.abs(want.astype(np.float64)).max(0)
     err = np.abs(got.astype(np.float64) - want.astype(np.float64)).max(0)
     assert (err <= TOL[dtype] * scale).all()
+
+
+def test_lines_fetched_ahead():
+    """K of 1.7 GB (from 1.5 GB on a group's lines are fetched ahead): K x as after the colour
+    schedule.  A row sums up to 8 element entries and then 243 products in FP32; its entries and x
+    are of order max |K x| / 1, so 300 roundings of it bound the difference."""
+    import ctypes as C
+
+    import torch
+    from gpufem_b200.fem import Context
+    m = mg.structured(mg.BRICK20, (52, 52, 52), jitter=0.05, seed=1, ngauss=2)
+    with Context(0) as ctx:
+        ctx.mesh_create(m.elem_type, m.coords, m.conn, m.ngauss, 210e3, None, 0.3)
+        x = torch.randn(m.ndof, generator=torch.Generator().manual_seed(3)).cuda()
+        ys = []
+        for scatter in (_lib.GF_SCATTER_COLOR, _lib.GF_SCATTER_ATOMIC):
+            ctx.assemble(_lib.GF_F32, scatter)
+            y = torch.empty_like(x)
+            _lib.check(_lib.lib.gf_spmv(ctx.h, _lib.GF_F32, C.c_void_p(x.data_ptr()),
+                                        C.c_void_p(y.data_ptr())), ctx.h)
+            ys.append(y.double())
+    assert float((ys[0] - ys[1]).abs().max()) <= 300 * 2.0**-24 * float(ys[0].abs().max())
