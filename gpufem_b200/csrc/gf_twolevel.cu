@@ -53,8 +53,11 @@ struct Coarse {
   int ntiles = 0;                 // nt (nt + 1) / 2 tiles (I <= J) of the symmetric inverse
   int2* tile_ij = nullptr;        // [ntiles] (I, J)
   double* ainv = nullptr;         // [ntiles][64][64], zero beyond nc
-  int parts = 1;                  // blocks per aggregate of the fused update
-  double* rc = nullptr;          // [parts][64 nt], partial sums of P^T r
+  int nblk = 0;                   // blocks of the fused update
+  int4* blk = nullptr;            // [nblk] aggregate, first node, end, row of rc + 256 blocks
+  int parts = 1;                  // rows of rc that hold the sums of an aggregate of mean size
+  uint8_t* shares = nullptr;      // [64 nt] rows of rc that an entry sums, if any more than parts
+  double* rc = nullptr;          // [most blocks of an aggregate][64 nt], partial sums of P^T r
   double* zc = nullptr;          // [64 nt]
 };
 
@@ -849,7 +852,7 @@ __device__ inline double warp_sum8(const double (&e)[8]) {
 // zc += Ainv rc from the packed upper-triangle tiles: block per tile (I, J) adds A_IJ rc_J
 // to zc_I and, off the diagonal, A_IJ^T rc_I to zc_J (double atomics; zc is zeroed by the
 // restriction), so the symmetric inverse is read once at half its size.  rc is the sum of
-// `parts` partial vectors of length ld.  Warp w reads rows 8w .. 8w+7 of the tile as 16-byte
+// `parts` partial vectors of length ld (of shares[j], if more and shares is given).  Warp w reads rows 8w .. 8w+7 of the tile as 16-byte
 // pairs, one contiguous 512-byte row per load (lane l: columns 2l, 2l+1), all in flight before
 // rc is looked at, and kept in L2 from one iteration to the next.  Column sums: per thread over
 // its 8 rows, then over the warps in shared memory.  With sc: the block adds its part of
@@ -857,8 +860,8 @@ __device__ inline double warp_sum8(const double (&e)[8]) {
 // zc by the last block to end took the kernel's tail (fence, counter, one block reading zc).
 __global__ void __launch_bounds__(256)
 k_coarse_symv(const int2* __restrict__ ij, const double* __restrict__ T,
-              const double* __restrict__ rc, int parts, int ld, double* __restrict__ zc,
-              SolveScalars* sc, const int* __restrict__ done) {
+              const double* __restrict__ rc, int parts, const uint8_t* __restrict__ shares, int ld,
+              double* __restrict__ zc, SolveScalars* sc, const int* __restrict__ done) {
   __shared__ double xI[kTS], xJ[kTS], colp[8][kTS], red[8];
   if (done && *done) return;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -869,9 +872,13 @@ k_coarse_symv(const int2* __restrict__ ij, const double* __restrict__ T,
   for (int c = 0; c < 8; ++c) a[c] = __ldg(base + c * 32 + lane);
   const int2 t = ij[blockIdx.x];
   if (tid < 2 * kTS) {
-    const double* src = rc + (tid < kTS ? t.x * kTS + tid : t.y * kTS + tid - kTS);
+    const int j = tid < kTS ? t.x * kTS + tid : t.y * kTS + tid - kTS;
+    const int more = shares ? shares[j] : 0;
+    const double* src = rc + j;
     double v = 0.0;
     for (int k = 0; k < parts; ++k) v += src[(int64_t)k * ld];
+#pragma unroll 8
+    for (int k = parts; k < more; ++k) v += src[(int64_t)k * ld];
     (tid < kTS ? xI[tid] : xJ[tid - kTS]) = v;
   }
   __syncthreads();
@@ -972,20 +979,23 @@ k_prolong(int n, const int32_t* __restrict__ agg, const double* __restrict__ x,
 
 // INIT: x = 0, r = scale * b.  Else: alpha = rz / p.q, x += alpha p, r -= alpha q.
 // Accumulates rr = r.r and rzn += r.D^-1 r (in FP64 whatever the vector type V), and restricts
-// r: every node is in one aggregate, so a block walks its share (blockIdx.y of gridDim.y) of
-// aggregate blockIdx.x's node list, updates those nodes' entries and leaves the share's sums of
-// P^T r in rc[blockIdx.y]; the block of share 0 zeroes the aggregate's part of zc for the
-// coarse product.  Bound by latency at the sizes where it matters (182k dofs: 1.4 MB per
-// vector, in L2), hence one thread per node with all of its entries' loads in flight, enough
-// shares per aggregate for one or two nodes per thread, and one warp reduction for the eight
-// sums.  As two kernels, x/r by rows and the restriction by a block per aggregate, it was a
-// launch and a second pass over r more.  An iteration with this, the coarse product's own r.z
-// and the direction per node: Brick20 24^3 FP64 64.2 -> 58.2 us, 14^3 26.7 -> 22.6, Q8 128
-// 23.3 -> 18.5; from 600k dofs on no difference.
-constexpr int kUT = 128;
+// r: every node is in one aggregate, so a block takes a share of an aggregate's node list
+// (blk[blockIdx.x]), updates those nodes' entries and leaves the share's sums of P^T r in its
+// row of rc; the block of row 0 zeroes the aggregate's part of zc for the coarse product.
+// Bound by latency at the sizes where it matters (182k dofs: 1.4 MB per vector, in L2), hence
+// one thread per node with all of its entries' loads in flight, shares of one or two nodes per
+// thread, and one warp reduction for the eight sums.  As two kernels, x/r by rows and the
+// restriction by a block per aggregate, it was a launch and a second pass over r more.  An
+// iteration with this, the coarse product's own r.z and the direction per node: Brick20 24^3
+// FP64 64.2 -> 58.2 us, 14^3 26.7 -> 22.6, Q8 128 23.3 -> 18.5; from 600k dofs on no difference.
+// On a graded mesh some boxes hold many times the mean, so the number of blocks goes by the
+// aggregate.  With the same number for all, the iteration waited for the largest: Brick8 40^3,
+// 64^3 with 73% of the nodes in one box 170, 802 us -> 58, 171 (uniform 43, 129); coordinates
+// cubed 92, 241 -> 51, 134; Q4 200^2 cubed 50 -> 26 (uniform 18.5).
+constexpr int kUT = 128, kMaxShares = 64;
 template <int DIM, bool INIT, typename V>
 __global__ void __launch_bounds__(kUT, 1)
-k_tl_update(const int32_t* __restrict__ off, const int32_t* __restrict__ nodes,
+k_tl_update(const int4* __restrict__ blk, const int32_t* __restrict__ nodes,
             const double* __restrict__ xc, const double* __restrict__ cen, double sinv,
             const uint8_t* __restrict__ fixed, const double* __restrict__ b,
             const V* __restrict__ q, double scale, V* __restrict__ x, V* __restrict__ r,
@@ -994,25 +1004,25 @@ k_tl_update(const int32_t* __restrict__ off, const int32_t* __restrict__ nodes,
   constexpr int NM = DIM == 2 ? 3 : 6;
   static_assert(NM + 2 <= 8, "sums per warp reduction");
   __shared__ double ws[kUT / 32][8];
+  const int4 share = __ldg(blk + blockIdx.x);   // on its way while the scalars are looked at
   double alpha = 0.0;
   if (!INIT) {
     if (sc->done) return;
     const double pq = sc->pq;
     if (!(pq > 0.0) || !isfinite(pq)) {
-      if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) sc->done = 2;
+      if (blockIdx.x == 0 && threadIdx.x == 0) sc->done = 2;
       return;
     }
     alpha = sc->rz / pq;
   }
-  const int A = blockIdx.x;
+  const int A = share.x, row = share.w & 255, stride = (share.w >> 8) * kUT;
   double cA[DIM];
 #pragma unroll
   for (int c = 0; c < DIM; ++c) cA[c] = cen[(int64_t)A * DIM + c];
   double acc[8];  // the modes, r.r, r.D^-1 r
 #pragma unroll
   for (int m = 0; m < 8; ++m) acc[m] = 0.0;
-  const int end = off[A + 1];
-  for (int t = off[A] + blockIdx.y * kUT + threadIdx.x; t < end; t += gridDim.y * kUT) {
+  for (int t = share.y + threadIdx.x; t < share.z; t += stride) {
     const int a = nodes[t];
     const int64_t i = (int64_t)a * DIM;
     double d[DIM], f[DIM];
@@ -1052,8 +1062,8 @@ k_tl_update(const int32_t* __restrict__ off, const int32_t* __restrict__ nodes,
 #pragma unroll
     for (int k = 0; k < kUT / 32; ++k) u += ws[k][m];
     if (m < NM) {
-      rc[(int64_t)blockIdx.y * ld + A * NM + m] = u;
-      if (blockIdx.y == 0) zc[A * NM + m] = 0.0;
+      rc[(int64_t)row * ld + A * NM + m] = u;
+      if (row == 0) zc[A * NM + m] = 0.0;
     } else {
       atomicAdd(m == NM ? &sc->rr : &sc->rzn, u);
     }
@@ -1122,6 +1132,8 @@ void coarse_release(gf_ctx* ctx, Coarse* c) {
   gf_pfree(ctx, c->cen);
   gf_pfree(ctx, c->ainv);
   gf_pfree(ctx, c->tile_ij);
+  gf_pfree(ctx, c->blk);
+  gf_pfree(ctx, c->shares);
   gf_pfree(ctx, c->rc);
   gf_pfree(ctx, c->zc);
 }
@@ -1205,7 +1217,6 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
   const int ld = nt * kTS;  // length of rc, zc
   C->nt = nt;
   C->ntiles = ntiles;
-  C->parts = std::max(1, std::min(gf_blocks(nnodes, kUT * na), 16 * ctx->sm_count / na));
   C->dim = dim; C->nm = nm; C->na = na; C->nc = nc; C->s = side;
   for (int c = 0; c < 3; ++c) { C->lo[c] = g.lo[c]; C->nb[c] = g.nb[c]; }
   double* d_Ac = nullptr;
@@ -1223,7 +1234,6 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
       (st = gf_palloc(ctx, &C->cen, (size_t)na * dim)) != GF_OK ||
       (st = gf_palloc(ctx, &C->ainv, (size_t)ntiles * kTS * kTS)) != GF_OK ||
       (st = gf_palloc(ctx, &C->tile_ij, (size_t)ntiles)) != GF_OK ||
-      (st = gf_palloc(ctx, &C->rc, (size_t)ld * C->parts)) != GF_OK ||
       (st = gf_palloc(ctx, &C->zc, (size_t)ld)) != GF_OK ||
       (st = gf_palloc(ctx, &d_Ac, (size_t)nc * nc)) != GF_OK ||
       (st = gf_palloc(ctx, &d_xp, (size_t)nt * kTT)) != GF_OK ||
@@ -1274,6 +1284,35 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
   GF_CUDA(ctx, cudaStreamSynchronize(s));
   int maxcnt = 1;
   for (int A = 0; A < na; ++A) maxcnt = std::max(maxcnt, hoff[A + 1] - hoff[A]);
+  // blocks of the fused update: a thread per node while there are no more than 16 blocks per SM
+  // (more start a second wave), an aggregate of up to 3/2 of the mean size as one of the mean,
+  // at most kMaxShares to an aggregate; the first blocks of all aggregates, then the second ones
+  const int mean = gf_blocks(nnodes, na);
+  C->parts = std::max(1, std::min(gf_blocks(mean, kUT), 16 * ctx->sm_count / na));
+  const int most = std::max(kUT, gf_blocks((int64_t)mean * 3, 2 * C->parts));
+  auto shares = [&](int cnt) {
+    return cnt <= most * C->parts ? C->parts : std::min(kMaxShares, gf_blocks(cnt, most));
+  };
+  const int rows = std::max(C->parts, shares(maxcnt));
+  std::vector<int4> hblk;
+  std::vector<uint8_t> hshares(ld, 0);
+  for (int y = 0; y < rows; ++y)
+    for (int A = 0; A < na; ++A) {
+      const int p = shares(hoff[A + 1] - hoff[A]);
+      if (y < p) hblk.push_back(make_int4(A, hoff[A] + y * kUT, hoff[A + 1], y | p << 8));
+      if (y == 0) std::fill_n(hshares.begin() + A * nm, nm, (uint8_t)p);
+    }
+  C->nblk = (int)hblk.size();
+  if ((st = gf_palloc(ctx, &C->blk, hblk.size())) != GF_OK ||
+      (rows > C->parts && (st = gf_palloc(ctx, &C->shares, (size_t)ld)) != GF_OK) ||
+      (st = gf_palloc(ctx, &C->rc, (size_t)ld * rows)) != GF_OK) {
+    cleanup2();
+    return st;
+  }
+  GF_CUDA(ctx, cudaMemcpyAsync(C->blk, hblk.data(), sizeof(int4) * hblk.size(),
+                               cudaMemcpyHostToDevice, s));
+  if (C->shares)
+    GF_CUDA(ctx, cudaMemcpyAsync(C->shares, hshares.data(), (size_t)ld, cudaMemcpyHostToDevice, s));
   const int per = (int)((maxcnt + (int64_t)kCMT * 65535 - 1) / ((int64_t)kCMT * 65535));
   const dim3 gcm(na, (maxcnt + kCMT * per - 1) / (kCMT * per));
   if (ctx->d_adj && ctx->d_adj_off && na < (1 << 24) && gf_sell_prepare(ctx, GF_F64) == GF_OK &&
@@ -1322,7 +1361,8 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
   }
   k_sweep_finish<<<ntiles, 256, 0, s>>>(nc, C->tile_ij, C->ainv);
   ctx->launches += 1 + 2 * (int64_t)nt;
-  cudaMemsetAsync(C->rc, 0, sizeof(double) * ld * C->parts, s);  // the tails beyond nc stay zero
+  // the tails beyond nc, and the rows beyond an aggregate's blocks, stay zero
+  cudaMemsetAsync(C->rc, 0, sizeof(double) * ld * rows, s);
   cudaMemsetAsync(C->zc, 0, sizeof(double) * ld, s);
   ctx->launches++;
   cudaError_t e = cudaStreamSynchronize(s);
@@ -1373,15 +1413,15 @@ static void coarse_apply_impl(gf_ctx* ctx, const double* r, const double* dinv, 
   if (c->dim == 2) {
     k_restrict<2><<<c->na, kRT, 0, s>>>(c->agg_off, c->agg_nodes, ctx->d_coords64, c->cen, sinv,
                                         ctx->d_fixed, r, c->rc, c->zc, done);
-    k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->tile_ij, c->ainv, c->rc, 1, 0, c->zc, nullptr,
-                                            done);
+    k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->tile_ij, c->ainv, c->rc, 1, nullptr, 0, c->zc,
+                                            nullptr, done);
     k_prolong<2><<<pb, kCT, 0, s>>>(ctx->n, c->node_agg, ctx->d_coords64, c->cen, sinv,
                                     ctx->d_fixed, dinv, r, c->zc, z, rz_acc, done, add);
   } else {
     k_restrict<3><<<c->na, kRT, 0, s>>>(c->agg_off, c->agg_nodes, ctx->d_coords64, c->cen, sinv,
                                         ctx->d_fixed, r, c->rc, c->zc, done);
-    k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->tile_ij, c->ainv, c->rc, 1, 0, c->zc, nullptr,
-                                            done);
+    k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->tile_ij, c->ainv, c->rc, 1, nullptr, 0, c->zc,
+                                            nullptr, done);
     k_prolong<3><<<pb, kCT, 0, s>>>(ctx->n, c->node_agg, ctx->d_coords64, c->cen, sinv,
                                     ctx->d_fixed, dinv, r, c->zc, z, rz_acc, done, add);
   }
@@ -1408,17 +1448,16 @@ static void tl_launch(gf_ctx* ctx, int mode, const double* b, const V* q, double
   const int grid = std::min(gf_blocks(nn, kCT), ctx->sm_count * 8);
   const uint8_t* fx = ctx->d_fixed;
   const double* xc = ctx->d_coords64;
-  const dim3 gu(c->na, c->parts);
   if (mode == kTlStep)
-    k_tl_update<DIM, false, V><<<gu, kUT, 0, s>>>(c->agg_off, c->agg_nodes, xc, c->cen, sinv, fx,
-                                                  nullptr, q, 1.0, x, r, p, dinv, c->rc, ld,
-                                                  c->zc, sc);
+    k_tl_update<DIM, false, V><<<c->nblk, kUT, 0, s>>>(c->blk, c->agg_nodes, xc, c->cen, sinv, fx,
+                                                       nullptr, q, 1.0, x, r, p, dinv, c->rc, ld,
+                                                       c->zc, sc);
   else
-    k_tl_update<DIM, true, V><<<gu, kUT, 0, s>>>(c->agg_off, c->agg_nodes, xc, c->cen, sinv, fx, b,
-                                                 nullptr, scale, x, r, nullptr, dinv, c->rc, ld,
+    k_tl_update<DIM, true, V><<<c->nblk, kUT, 0, s>>>(c->blk, c->agg_nodes, xc, c->cen, sinv, fx, b,
+                                                      nullptr, scale, x, r, nullptr, dinv, c->rc, ld,
                                                  c->zc, sc);
-  k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->tile_ij, c->ainv, c->rc, c->parts, ld, c->zc, sc,
-                                          &sc->done);
+  k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->tile_ij, c->ainv, c->rc, c->parts, c->shares, ld,
+                                          c->zc, sc, &sc->done);
   auto* direction = mode == kTlFirst  ? k_tl_direction<DIM, kTlFirst, V>
                     : mode == kTlKeep ? k_tl_direction<DIM, kTlKeep, V>
                                       : k_tl_direction<DIM, kTlStep, V>;
