@@ -59,6 +59,7 @@ struct MatLayout {
   int nnodes = 0;
   const int32_t* __restrict__ perm = nullptr;  // node-block slices: node of each slot
   int split = 1;  // node-block slices: warps that share a slice (slice_split)
+  bool one_slot = false;  // 3-D, two warps: one neighbour slot in flight (one_slot)
 
   __device__ inline bool at(int t, int& nz, int64_t& o, int64_t& stride) const {
     if (t >= count) return false;
@@ -130,6 +131,7 @@ __device__ inline void ldg_pair(const double* __restrict__ x, int b, Acc& x0, Ac
 // ELL / SELL: a thread per row, rows strided over a capped grid.
 struct RowWalk {
   static constexpr int kThreads = kT;
+  static constexpr int kBlocks64 = 1;
   static int grid(const gf_ctx* ctx, const MatLayout& L) {
     return std::min(gf_blocks(L.count, kThreads), ctx->sm_count * 8);
   }
@@ -162,13 +164,18 @@ struct RowWalk {
 // 128 PCG FP64 13.5 -> 12.4 us an iteration, 12.9 with one and 14.7 with four).  Whole PCG
 // iterations in FP64: Brick20 14^3 38.5 -> 16.7 us, 24^3 59.4 -> 49.4, 32^3 108 -> 101, Brick8
 // 30^3 22.4 -> 16.9, 64^3 99.0 -> 98.8.
-// Eight warps per slice, four slots in flight, blocks of 64, launch bounds that force more warps
-// per SM, and a bulk prefetch of the slice into L2 all measured slower.  The bounds name one
-// block per SM: without it the compiler aims at 32 registers, which serialises a slot's loads
-// (Brick20 24^3 FP64 52 -> 71 us).
+// Eight warps per slice, four slots in flight, blocks of 64, and a bulk prefetch of the slice into
+// L2 all measured slower.  The launch bounds name one block per SM: without it the compiler aims at
+// 32 registers, which serialises a slot's loads (Brick20 24^3 FP64 52 -> 71 us).
+// Two slots in flight take 122 registers in FP64, four blocks (eight slices) to an SM; a matrix
+// with more slices than that takes one slot and 64 registers, eight blocks.  Brick8 FP64 PCG, us
+// an iteration with two slots, with one, and with one warp per slice: 20^3 12.8, 14.2, 17.9; 32^3
+// (7.6 slices per SM) 20.3, 20.8, 25.0; 40^3 34.0, 33.1, 34.4; 64^3 99.7, 99.2, 100.1; 112^3
+// 519.7, 508.7, 510.5; 128^3 771.7, 752.1, 753.1.
 template <int DIM, int SPLIT, int UN>
 struct NodeWalk {
   static constexpr int kThreads = 128;
+  static constexpr int kBlocks64 = DIM == 3 && SPLIT == 2 && UN == 1 ? 8 : 1;  // per SM, in FP64
   static constexpr int kSlices = kThreads / 32 / SPLIT;  // per block
   static int grid(const gf_ctx*, const MatLayout& L) {
     return gf_blocks(gf_blocks(L.nnodes, 32), kSlices);
@@ -267,9 +274,17 @@ inline int slice_split(const gf_ctx* ctx, int dim, int nnodes, int64_t slots) {
   return nslice <= 16 * (int64_t)ctx->sm_count ? 2 : 1;
 }
 
-// Calls g(walk) with the policy of layout L.
-template <typename G>
-inline void with_walk(const MatLayout& L, G&& g) {
+inline bool one_slot(const gf_ctx* ctx, int dim, int split, int dtype, int nnodes) {
+  return dim == 3 && split == 2 && dtype == GF_F64 &&
+         gf_blocks(nnodes, 32) > 8 * (int64_t)ctx->sm_count;
+}
+
+// Calls g(walk) with the policy of layout L for a matrix of type TK.
+template <typename TK, typename G>
+inline void with_walk(const MatLayout& L, const TK*, G&& g) {
+  if constexpr (sizeof(TK) == 8) {
+    if (L.one_slot) return g(NodeWalk<3, 2, 1>{});
+  }
   if (L.bdim == 2)
     L.split == 1 ? g(NodeWalk<2, 1, 1>{}) : g(NodeWalk<2, 2, 1>{});
   else if (L.bdim == 3)
@@ -278,16 +293,17 @@ inline void with_walk(const MatLayout& L, G&& g) {
     g(RowWalk{});
 }
 
-// launches the kernel (in parentheses, a template over `Walk`) over the rows of L on stream s
-#define GF_ROWS_LAUNCH(ctx, s, L, KERNEL, ...)                                    \
-  with_walk(L, [&](auto walk) {                                                   \
-    using Walk = decltype(walk);                                                  \
-    GF_UNPAREN KERNEL<<<Walk::grid(ctx, L), Walk::kThreads, 0, s>>>(L, __VA_ARGS__); \
+// launches the kernel (in parentheses, a template over `Walk`) over the rows of L, whose values
+// are `val`, on stream s
+#define GF_ROWS_LAUNCH(ctx, s, L, KERNEL, val, ...)                                    \
+  with_walk(L, val, [&](auto walk) {                                                   \
+    using Walk = decltype(walk);                                                       \
+    GF_UNPAREN KERNEL<<<Walk::grid(ctx, L), Walk::kThreads, 0, s>>>(L, val, __VA_ARGS__); \
   })
 #define GF_UNPAREN(...) __VA_ARGS__
 
 template <class W, typename TK, typename TX, typename TY>
-__global__ void __launch_bounds__(W::kThreads, 1)
+__global__ void __launch_bounds__(W::kThreads, sizeof(TK) == 8 || sizeof(TX) == 8 ? W::kBlocks64 : 1)
 k_spmv(MatLayout L, const TK* __restrict__ val, const TX* __restrict__ x, TY* __restrict__ y) {
   W::rows(L, val, x, [&](int row, double v) { y[row] = (TY)v; });
 }
@@ -295,7 +311,7 @@ k_spmv(MatLayout L, const TK* __restrict__ val, const TX* __restrict__ x, TY* __
 // y = scale .* (K x) for FP32 x and y (scale may be null), FP64 accumulation with FP64
 // values
 template <class W, typename TK>
-__global__ void __launch_bounds__(W::kThreads, 1)
+__global__ void __launch_bounds__(W::kThreads, sizeof(TK) == 8 ? W::kBlocks64 : 1)
 k_spmv_rowscale(MatLayout L, const TK* __restrict__ val, const float* __restrict__ x,
                 const float* __restrict__ scale, float* __restrict__ y) {
   W::rows(L, val, x, [&](int row, double v) {
@@ -305,7 +321,7 @@ k_spmv_rowscale(MatLayout L, const TK* __restrict__ val, const float* __restrict
 
 // r = f - K u (FP64), and r.r
 template <class W>
-__global__ void __launch_bounds__(W::kThreads, 1)
+__global__ void __launch_bounds__(W::kThreads, W::kBlocks64)
 k_residual64(MatLayout L, const double* __restrict__ val, const double* __restrict__ u,
              const double* __restrict__ f, double* __restrict__ r, double* __restrict__ acc) {
   __shared__ double sh[32];
@@ -390,7 +406,7 @@ __global__ void k_cg_init_fin(SolveScalars* sc, double eps, int maxit) {
 }
 
 template <class W, typename TK, typename V>
-__global__ void __launch_bounds__(W::kThreads, 1)
+__global__ void __launch_bounds__(W::kThreads, sizeof(TK) == 8 || sizeof(V) == 8 ? W::kBlocks64 : 1)
 k_cg_spmv_dot(MatLayout L, const TK* __restrict__ val, const V* __restrict__ p,
               V* __restrict__ q, SolveScalars* sc) {
   __shared__ double sh[32];
@@ -599,6 +615,7 @@ gf_status solver_matrix(gf_ctx* ctx, int dtype, MatLayout* L, const void** val) 
     L->nnodes = ctx->nnodes;
     L->perm = ctx->d_sell_perm;
     L->split = slice_split(ctx, L->bdim, L->nnodes, ctx->sell_total / 32);
+    L->one_slot = one_slot(ctx, L->bdim, L->split, dtype, L->nnodes);
   }
   *val = dtype == GF_F64 ? (const void*)ctx->d_sell_v64 : (const void*)ctx->d_sell_v32;
   return GF_OK;
@@ -1180,7 +1197,7 @@ __global__ void k_fcg_dir(int n, const double* __restrict__ z, double* __restric
 }
 
 template <class W>
-__global__ void __launch_bounds__(W::kThreads, 1)
+__global__ void __launch_bounds__(W::kThreads, W::kBlocks64)
 k_fcg_spmv(MatLayout L, const double* __restrict__ val, const double* __restrict__ p,
            const double* __restrict__ r, double* __restrict__ q, FcgScalars* sc) {
   __shared__ double sh[32];
@@ -1723,7 +1740,7 @@ __global__ void k_dist_scatter(int m, const int32_t* __restrict__ idx, const dou
 // q = K_local p over every local row; p.q over the owned rows only.  Block 0 clears the
 // r.z / r.r slots that the update kernel accumulates into next.
 template <class W>
-__global__ void __launch_bounds__(W::kThreads, 1)
+__global__ void __launch_bounds__(W::kThreads, W::kBlocks64)
 k_dist_spmv_dot(MatLayout L, const double* __restrict__ val, const double* __restrict__ p,
                 double* __restrict__ q, int no, DistScalars* sc) {
   __shared__ double sh[32];
