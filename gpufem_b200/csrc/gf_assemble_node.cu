@@ -22,13 +22,19 @@ namespace {
 
 // ---------------------------------------------------------------------------
 // Geometry layout.  An element's values (per Gauss point J^-1 row by row, then w detJ E) form
-// 16-byte units; eight consecutive elements interleave their units, so that the lanes of a
-// warp, whose nodes mostly walk consecutive elements, read whole 128-byte lines: unit u of
-// element e is at 16-byte index ((e / 8) * units + u) * 8 + e % 8.  (An element's block in
-// one piece costs a warp a line per lane and load: with such blocks the Q8 kernel below took
-// 157 us on 512 x 512 instead of 144.)  In 3-D each layer of Gauss points (first natural
+// 16-byte units.  Where consecutive nodes lie in elements of like numbers, IL = 8 consecutive
+// elements interleave their units, so that the lanes of a warp, whose nodes walk those elements,
+// read whole 128-byte lines: unit u of element e is at 16-byte index ((e / 8) * units + u) * 8 +
+// e % 8.  On a scattered numbering (gf_ctx::scattered) a lane would read a sector and a line for
+// each 16 bytes: there an element's units lie in one piece (IL = 1), whose sectors the lane uses
+// whole.  Us per call with IL = 8 and 1, by the share of distinct groups of eight among the
+// elements of 32 consecutive nodes (FP32; FP64):
+//   Q8 512^2     0.11 164, 200; 316, 362   0.34 204, 202; 390, 369   1 296, 229; 709, 424
+//   Q4 1024^2    0.15 130, 143; 205, 247   0.36 159, 156; 274, 282   1 281, 197; 503, 323
+//   Brick8 80^3  0.15 425, 565; 1008, 1273 0.36 854, 690; 1722, 1598 1 2098, 784; 4373, 1634
+// (0.27: Brick8 667, 600; 1373, 1434.)  In 3-D each layer of Gauss points (first natural
 // coordinate) is padded to whole units.
-template <int ET, typename T, int NG1>
+template <int ET, typename T, int NG1, int IL>
 struct Geo {
   static constexpr int DIM = gf_elem_info(ET).dim, GV = DIM * DIM + 1;
   static constexpr int U = 16 / (int)sizeof(T);                         // values per unit
@@ -36,7 +42,14 @@ struct Geo {
   static constexpr int PER = NG1 * NG1 * GV;                            // values per layer
   static constexpr int LU = (PER + U - 1) / U;                          // units per layer
   static constexpr int UNITS = LAYERS * LU;
-  static constexpr size_t bytes(int nelem) { return (size_t)((nelem + 7) / 8) * 8 * UNITS * 16; }
+  static constexpr size_t bytes(int nelem) { return (size_t)((nelem + IL - 1) / IL) * IL * UNITS * 16; }
+  // unit 0 of element e; its other units are IL further on each
+  template <typename P>
+  __device__ __forceinline__ static P* at(P* geo, int e) {
+    static_assert(IL == 1 || IL == 8, "shifts");
+    if constexpr (IL == 1) return geo + (int64_t)e * UNITS;
+    return geo + (int64_t)(e >> 3) * (UNITS * 8) + (e & 7);
+  }
 };
 
 template <typename T> struct Unit;
@@ -78,10 +91,10 @@ __device__ __forceinline__ R point_geometry(int g, const R (&X)[NEN][DIM], T Ee,
 }
 
 // All Gauss points of one element in R arithmetic; returns whether max/min |detJ| > 10.
-template <int ET, typename T, int NG1, typename R, int NEN, int DIM>
+template <int ET, typename T, int NG1, int IL, typename R, int NEN, int DIM>
 __device__ __forceinline__ bool element_geometry(const R (&X)[NEN][DIM], T Ee,
                                                  typename Unit<T>::type* out) {
-  using G = Geo<ET, T, NG1>;
+  using G = Geo<ET, T, NG1, IL>;
   R dmin = R(3.4e38), dmax = R(0);
 #pragma unroll
   for (int l = 0; l < G::LAYERS; ++l) {
@@ -96,26 +109,22 @@ __device__ __forceinline__ bool element_geometry(const R (&X)[NEN][DIM], T Ee,
       // the units that this point completes
 #pragma unroll
       for (int u = g * G::GV / G::U; u < ((g + 1) * G::GV) / G::U; ++u)
-        unit_put(out + (l * G::LU + u) * 8, buf + u * G::U);
+        unit_put(out + (l * G::LU + u) * IL, buf + u * G::U);
     }
     if constexpr (G::PER % G::U != 0)
-      unit_put(out + (l * G::LU + G::LU - 1) * 8, buf + (G::LU - 1) * G::U);
+      unit_put(out + (l * G::LU + G::LU - 1) * IL, buf + (G::LU - 1) * G::U);
   }
   return dmax > R(10) * dmin;
 }
 
 constexpr int kGT = 128;
 
-// A thread per element: its local coordinates stay in registers and the Gauss rule is a
-// compile-time table; the stores of a warp are whole lines by the layout.
-template <int ET, typename T, int NG1>
-__global__ void __launch_bounds__(kGT)
-k_geometry(int nelem, const int32_t* __restrict__ conn, const double* __restrict__ coords,
-           const T* __restrict__ Eel, T* __restrict__ geo) {
-  using G = Geo<ET, T, NG1>;
+// Geometry of element e to `out` (its unit 0).
+template <int ET, typename T, int NG1, int IL>
+__device__ __forceinline__ void one_element(int e, const int32_t* __restrict__ conn,
+                                            const double* __restrict__ coords,
+                                            const T* __restrict__ Eel, typename Unit<T>::type* out) {
   constexpr int NEN = gf_elem_info(ET).nen, DIM = gf_elem_info(ET).dim;
-  const int e = blockIdx.x * kGT + threadIdx.x;
-  if (e >= nelem) return;
   double X[NEN][DIM];
   double x0[DIM];
 #pragma unroll
@@ -129,16 +138,40 @@ k_geometry(int nelem, const int32_t* __restrict__ conn, const double* __restrict
     }
   }
   const T Ee = __ldg(Eel + e);
-  auto* out = reinterpret_cast<typename Unit<T>::type*>(geo) + (int64_t)(e >> 3) * (G::UNITS * 8) + (e & 7);
   if constexpr (sizeof(T) == 4) {
     float Xf[NEN][DIM];
 #pragma unroll
     for (int i = 0; i < NEN; ++i)
 #pragma unroll
       for (int c = 0; c < DIM; ++c) Xf[i][c] = (float)X[i][c];
-    if (!element_geometry<ET, T, NG1, float>(Xf, Ee, out)) return;
+    if (!element_geometry<ET, T, NG1, IL, float>(Xf, Ee, out)) return;
   }
-  element_geometry<ET, T, NG1, double>(X, Ee, out);
+  element_geometry<ET, T, NG1, IL, double>(X, Ee, out);
+}
+
+// A thread per element: its local coordinates stay in registers and the Gauss rule is a
+// compile-time table.  With IL = 8 the stores of a warp are whole lines by the layout; with IL = 1
+// they pass through shared memory where the block's units fit 48 KB (all but FP64 Brick8 and
+// Brick8 with 3^3 points): Q8 512^2 FP64 397 -> 362 us the assembly, Brick8 80^3 FP32 592 -> 565.
+template <int ET, typename T, int NG1, int IL>
+__global__ void __launch_bounds__(kGT)
+k_geometry(int nelem, const int32_t* __restrict__ conn, const double* __restrict__ coords,
+           const T* __restrict__ Eel, T* __restrict__ geo) {
+  using G = Geo<ET, T, NG1, IL>;
+  using UT = typename Unit<T>::type;
+  constexpr int ROW = G::UNITS | 1;   // units of an element in shared memory
+  constexpr bool kStage = IL == 1 && kGT * ROW * 16 <= 48 * 1024;
+  __shared__ UT stage[kStage ? kGT * ROW : 1];
+  const int e0 = blockIdx.x * kGT, e = e0 + threadIdx.x;
+  UT* all = reinterpret_cast<UT*>(geo);
+  if (e < nelem)
+    one_element<ET, T, NG1, IL>(e, conn, coords, Eel, kStage ? stage + threadIdx.x * ROW : G::at(all, e));
+  if constexpr (kStage) {
+    __syncthreads();
+    const int cnt = min(kGT, nelem - e0) * G::UNITS;
+    for (int k = threadIdx.x; k < cnt; k += kGT)
+      all[(int64_t)e0 * G::UNITS + k] = stage[k / G::UNITS * ROW + k % G::UNITS];
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -167,13 +200,13 @@ size_t node_rows_2d_smem(int W) {
          sizeof(int) * (3 * NB + 1 + (NB / 32 + 1) * kDegBuckets);
 }
 
-template <int ET, typename T, int NG1, int NB>
+template <int ET, typename T, int NG1, int IL, int NB>
 __global__ void __launch_bounds__(NB)
 k_node_rows_2d(int nnodes, int n, int W, const int32_t* __restrict__ inc_off,
                const int32_t* __restrict__ inc, const uint8_t* __restrict__ inc_loc,
                const uint16_t* __restrict__ inc_slot, const T* __restrict__ geo,
                const AsmTables* __restrict__ tab, T lam1, T mu1, T* __restrict__ K) {
-  using G = Geo<ET, T, NG1>;
+  using G = Geo<ET, T, NG1, IL>;
   using T2 = typename Vec2<T>::type;
   using UT = typename Unit<T>::type;
   constexpr int NEN = gf_elem_info(ET).nen, NGP = NG1 * NG1, RB = 2 * NB, NW = NB / 32;
@@ -254,7 +287,7 @@ k_node_rows_2d(int nnodes, int n, int W, const int32_t* __restrict__ inc_off,
     const int64_t q = q0 + k;
     const int e = __ldg(inc + q);
     i = __ldg(inc_loc + q);
-    ge = reinterpret_cast<const UT*>(geo) + (int64_t)(e >> 3) * (G::UNITS * 8) + (e & 7);
+    ge = G::at(reinterpret_cast<const UT*>(geo), e);
     if constexpr (NEN == 8) {
       const uint4 v = __ldg(reinterpret_cast<const uint4*>(inc_slot + q * NEN));
       sn[0] = v.x; sn[1] = v.y; sn[2] = v.z; sn[3] = v.w;
@@ -266,7 +299,7 @@ k_node_rows_2d(int nnodes, int n, int W, const int32_t* __restrict__ inc_off,
   if (deg > 0) {
     meta(0);
 #pragma unroll
-    for (int u = 0; u < G::UNITS; ++u) unit_get(__ldg(ge + u * 8), gv + u * G::U);
+    for (int u = 0; u < G::UNITS; ++u) unit_get(__ldg(ge + u * IL), gv + u * G::U);
   }
   for (int k = 0; k < deg; ++k) {
     const T2* dn_i = sdN + i;
@@ -303,7 +336,7 @@ k_node_rows_2d(int nnodes, int n, int W, const int32_t* __restrict__ inc_off,
         const int to = g == NGP - 1 ? G::UNITS : (g + 1) * 5 / G::U;
         if (more)
 #pragma unroll
-          for (int u = from; u < to; ++u) unit_get(__ldg(ge + u * 8), gv + u * G::U);
+          for (int u = from; u < to; ++u) unit_get(__ldg(ge + u * IL), gv + u * G::U);
       }
     }
     // V = lam1 H + mu1 H^T + mu1 tr(H) I; column b of V is rows (2 al, 2 al + 1) of tile
@@ -387,13 +420,13 @@ size_t node_rows_b8_smem(int W) {
 
 // A lane per node, a warp (= CTA) per NB consecutive nodes, each lane's three rows in its own
 // columns of the tile [slot][3 NB] (no conflicts where the lanes' slots agree).
-template <typename T, int NG1>
+template <typename T, int NG1, int IL>
 __global__ void __launch_bounds__(32)
 k_node_rows_b8(int nnodes, int n, int W, const int32_t* __restrict__ inc_off,
                const int32_t* __restrict__ inc, const uint8_t* __restrict__ inc_loc,
                const uint16_t* __restrict__ inc_slot, const T* __restrict__ geo,
                const AsmTables* __restrict__ tab, T lam1, T mu1, T* __restrict__ K) {
-  using G = Geo<GF_BRICK8, T, NG1>;
+  using G = Geo<GF_BRICK8, T, NG1, IL>;
   using UT = typename Unit<T>::type;
   using T2 = typename Vec2<T>::type;
   constexpr int NB = b8_nodes<T>(), RB = 3 * NB, NGP = NG1 * NG1 * NG1, LP = NG1 * NG1;
@@ -436,13 +469,13 @@ k_node_rows_b8(int nnodes, int n, int W, const int32_t* __restrict__ inc_off,
     const int e = __ldg(inc + q);
     i = __ldg(inc_loc + q);
     sn = __ldg(reinterpret_cast<const uint4*>(inc_slot + q * 8));
-    ge = reinterpret_cast<const UT*>(geo) + (int64_t)(e >> 3) * (G::UNITS * 8) + (e & 7);
+    ge = G::at(reinterpret_cast<const UT*>(geo), e);
   };
   auto fetch = [&](int c) {
     const int l = c / CL, m = c % CL;
 #pragma unroll
     for (int u = 0; u < 5; ++u)
-      if (m * 5 + u < G::LU) gv[c % RC][u] = __ldg(ge + (l * G::LU + m * 5 + u) * 8);
+      if (m * 5 + u < G::LU) gv[c % RC][u] = __ldg(ge + (l * G::LU + m * 5 + u) * IL);
   };
   if (deg > 0) {
     meta(0);
@@ -577,20 +610,22 @@ k_node_rows_b8(int nnodes, int n, int W, const int32_t* __restrict__ inc_off,
 // ---------------------------------------------------------------------------
 constexpr size_t kNodeSmem = 56 * 1024;
 
-template <int ET, typename T, int NG1>
-gf_status launch_geometry(gf_ctx* ctx, T* geo) {
+template <int ET, typename T, int NG1, int IL>
+gf_status launch_geometry(gf_ctx* ctx) {
   const T* Eel = sizeof(T) == 8 ? (const T*)ctx->d_Eel : (const T*)ctx->d_Eel32;
-  k_geometry<ET, T, NG1><<<gf_blocks(ctx->nelem, kGT), kGT, 0, ctx->stream>>>(
-      ctx->nelem, ctx->d_conn, ctx->d_coords64, Eel, geo);
+  gf_status st = gf_geo_buffer(ctx, Geo<ET, T, NG1, IL>::bytes(ctx->nelem));
+  if (st != GF_OK) return st;
+  k_geometry<ET, T, NG1, IL><<<gf_blocks(ctx->nelem, kGT), kGT, 0, ctx->stream>>>(
+      ctx->nelem, ctx->d_conn, ctx->d_coords64, Eel, (T*)ctx->d_geo);
   GF_LAUNCH_CHECK(ctx, "k_geometry");
   cudaEventRecord(ctx->evm, ctx->stream);
   return GF_OK;
 }
 
-template <int ET, typename T, int NG1, int NB>
+template <int ET, typename T, int NG1, int IL, int NB>
 gf_status launch_2d(gf_ctx* ctx, T* K, const AsmTables* d_tab) {
   const size_t sm = node_rows_2d_smem<ET, T, NG1, NB>(ctx->W);
-  auto kern = k_node_rows_2d<ET, T, NG1, NB>;
+  auto kern = k_node_rows_2d<ET, T, NG1, IL, NB>;
   GF_CUDA(ctx, gf_smem_attr(kern, sm));
   kern<<<(ctx->nnodes + NB - 1) / NB, NB, sm, ctx->stream>>>(
       ctx->nnodes, ctx->n, ctx->W, ctx->d_inc_off, ctx->d_inc, ctx->d_inc_loc, ctx->d_inc_slot,
@@ -601,23 +636,23 @@ gf_status launch_2d(gf_ctx* ctx, T* K, const AsmTables* d_tab) {
 
 // Blocks of 128 nodes while four CTAs fit an SM and every SM gets one; smaller blocks for wider
 // rows (FP64 Q8: 64) and smaller meshes.
-template <int ET, typename T, int NG1>
+template <int ET, typename T, int NG1, int IL>
 gf_status assemble_2d(gf_ctx* ctx, T* K, const AsmTables* d_tab) {
-  gf_status st = gf_geo_buffer(ctx, Geo<ET, T, NG1>::bytes(ctx->nelem));
-  if (st != GF_OK || (st = launch_geometry<ET, T, NG1>(ctx, (T*)ctx->d_geo)) != GF_OK) return st;
+  gf_status st = launch_geometry<ET, T, NG1, IL>(ctx);
+  if (st != GF_OK) return st;
   if (node_rows_2d_smem<ET, T, NG1, 128>(ctx->W) <= kNodeSmem && ctx->nnodes >= 128 * ctx->sm_count)
-    return launch_2d<ET, T, NG1, 128>(ctx, K, d_tab);   // four or five CTAs per SM
+    return launch_2d<ET, T, NG1, IL, 128>(ctx, K, d_tab);   // four or five CTAs per SM
   if (node_rows_2d_smem<ET, T, NG1, 64>(ctx->W) <= kNodeSmem && ctx->nnodes >= 64 * ctx->sm_count)
-    return launch_2d<ET, T, NG1, 64>(ctx, K, d_tab);
-  return launch_2d<ET, T, NG1, 32>(ctx, K, d_tab);
+    return launch_2d<ET, T, NG1, IL, 64>(ctx, K, d_tab);
+  return launch_2d<ET, T, NG1, IL, 32>(ctx, K, d_tab);
 }
 
-template <typename T, int NG1>
+template <typename T, int NG1, int IL>
 gf_status assemble_b8(gf_ctx* ctx, T* K, const AsmTables* d_tab) {
-  gf_status st = gf_geo_buffer(ctx, Geo<GF_BRICK8, T, NG1>::bytes(ctx->nelem));
-  if (st != GF_OK || (st = launch_geometry<GF_BRICK8, T, NG1>(ctx, (T*)ctx->d_geo)) != GF_OK) return st;
+  gf_status st = launch_geometry<GF_BRICK8, T, NG1, IL>(ctx);
+  if (st != GF_OK) return st;
   const size_t sm = node_rows_b8_smem<T, NG1>(ctx->W);
-  auto kern = k_node_rows_b8<T, NG1>;
+  auto kern = k_node_rows_b8<T, NG1, IL>;
   GF_CUDA(ctx, gf_smem_attr(kern, sm));
   constexpr int NB = b8_nodes<T>();
   kern<<<(ctx->nnodes + NB - 1) / NB, 32, sm, ctx->stream>>>(
@@ -627,14 +662,20 @@ gf_status assemble_b8(gf_ctx* ctx, T* K, const AsmTables* d_tab) {
   return GF_OK;
 }
 
-template <typename T>
+template <typename T, int NG1, int IL>
 gf_status node_dispatch(gf_ctx* ctx, T* K, const AsmTables* d_tab) {
-  const bool two = ctx->ngauss == 2;
   switch (ctx->elem_type) {
-    case GF_Q4: return two ? assemble_2d<GF_Q4, T, 2>(ctx, K, d_tab) : assemble_2d<GF_Q4, T, 3>(ctx, K, d_tab);
-    case GF_Q8: return two ? assemble_2d<GF_Q8, T, 2>(ctx, K, d_tab) : assemble_2d<GF_Q8, T, 3>(ctx, K, d_tab);
-    default: return two ? assemble_b8<T, 2>(ctx, K, d_tab) : assemble_b8<T, 3>(ctx, K, d_tab);
+    case GF_Q4: return assemble_2d<GF_Q4, T, NG1, IL>(ctx, K, d_tab);
+    case GF_Q8: return assemble_2d<GF_Q8, T, NG1, IL>(ctx, K, d_tab);
+    default: return assemble_b8<T, NG1, IL>(ctx, K, d_tab);
   }
+}
+
+template <typename T>
+gf_status node_assemble(gf_ctx* ctx, T* K, const AsmTables* d_tab) {
+  if (ctx->scattered)
+    return ctx->ngauss == 2 ? node_dispatch<T, 2, 1>(ctx, K, d_tab) : node_dispatch<T, 3, 1>(ctx, K, d_tab);
+  return ctx->ngauss == 2 ? node_dispatch<T, 2, 8>(ctx, K, d_tab) : node_dispatch<T, 3, 8>(ctx, K, d_tab);
 }
 
 }  // namespace
@@ -665,6 +706,6 @@ bool gf_assemble_node_fits(const gf_ctx* ctx, int dtype) {
 
 // Launches the assembly on the context's stream (no sync).
 gf_status gf_assemble_node(gf_ctx* ctx, int dtype, const AsmTables* d_tab) {
-  if (dtype == GF_F64) return node_dispatch<double>(ctx, ctx->d_K64, d_tab);
-  return node_dispatch<float>(ctx, ctx->d_K32, d_tab);
+  if (dtype == GF_F64) return node_assemble(ctx, ctx->d_K64, d_tab);
+  return node_assemble(ctx, ctx->d_K32, d_tab);
 }

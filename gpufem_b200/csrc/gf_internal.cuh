@@ -239,6 +239,7 @@ struct gf_ctx {
   uint16_t* d_inc_slot = nullptr; // [incidence][nen]: neighbour position of each element node
   int32_t* d_einc = nullptr;      // [nelem][nen] incidence of each element node (Brick20 atomic)
   int maxval = 0;                 // max elements sharing one node
+  bool scattered = false;         // consecutive nodes lie in elements of unlike numbers
   void* d_geo = nullptr;          // owner scatter: J^-1, w detJ (E) per (element, Gauss point)
   size_t geo_bytes = 0;
 
