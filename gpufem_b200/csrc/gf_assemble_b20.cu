@@ -10,8 +10,8 @@
 // lanes (element, row): the rows of neighbouring elements' nodes lie 12 or 24 bytes apart in
 // a column of the ELL, so the lanes share lines.  Now L2 takes 140-150 G sectors of reductions
 // a second that miss it (1300 sectors per FP32 element; DRAM reads and writes K once), whatever
-// the order of the elements; from 52^3 (FP32) that is all that is left of the time, and the
-// lines are fetched to L2 ahead of the reductions.
+// the order of the elements; from 52^3 (FP32) that is all that is left of the time, and where the
+// mesh is ordered the lines are fetched to L2 ahead of the reductions.
 //   us, against a thread per node pair:    FP32  FP64
 //   Brick20   8^3                    32 -> 26   35 -> 30
 //   Brick20  24^3                  191 -> 160  375 -> 277
@@ -411,10 +411,14 @@ gf_status launch_b20(gf_ctx* ctx, const AsmTables* d_tab, T* K) {
   GF_CUDA(ctx, gf_smem_attr(kern, L::bytes));
   const T* Eel = sizeof(T) == 8 ? (const T*)ctx->d_Eel : (const T*)ctx->d_Eel32;
   const int groups = (ctx->nelem + L::E - 1) / L::E;
-  // from 1.5 GB of K on, reductions find their lines slower than L2 takes them (FP32 52^3 1605 ->
-  // 1499 us with the lines fetched ahead, 64^3 3247 -> 2959, FP64 44^3 1930 -> 1831); below, the
-  // extra requests cost (FP32 48^3 1032 -> 1176; FP64 36^3 900 -> 896)
-  const bool ahead = (int64_t)ctx->n * ctx->W * (int64_t)sizeof(T) > 1500000000;
+  // Lines fetched ahead on large matrices of ordered meshes.  Us with and without, FP32: 44^3 (1.0
+  // GB of K) 926, 952; 48^3 1197, 1113; 50^3 (1.5 GB) 1349, 1376; 52^3 1519, 1651; 64^3 3088, 3320;
+  // FP64: 28^3 446, 433; 32^3 642, 618; 38^3 (1.4 GB) 1052, 1191; 44^3 1915, 1990; 60^3 5137, 5288;
+  // 64^3 6573, 6552.  What a prefetch brings is a line; where the rows of consecutive elements'
+  // nodes do not fill the lines in order, most of it is fetched for nothing, and twice: FP32 56^3
+  // with the nodes shuffled in runs of 128, 16, 1 3128, 7372, 13869 against 2544, 4303, 9451, rows
+  // of 8 elements (8 x 8 x 3200) 2964 against 2412, of 16 2521 against 2451, of 52 1819 against 2047.
+  const bool ahead = ctx->consecutive && (int64_t)ctx->n * ctx->W * (int64_t)sizeof(T) > 1500000000;
   kern<<<std::min(groups, ctx->sm_count * 2), L::THREADS, L::bytes, ctx->stream>>>(
       ctx->nelem, ctx->n, ctx->d_conn, ctx->d_coords64, Eel, ctx->d_einc, ctx->d_inc_slot, d_tab,
       T(ctx->lam1), T(ctx->mu1), ahead, K);
