@@ -152,7 +152,8 @@ void gf_pattern_free(gf_ctx* ctx) {
   gf_pfree(ctx, ctx->d_inc_loc);
   gf_pfree(ctx, ctx->d_inc_slot);
   gf_pfree(ctx, ctx->d_einc);
-  ctx->maxval = 0;  // the geometry buffer keeps its capacity (freed by gf_destroy)
+  ctx->maxval = 0;  // the geometry buffer keeps its capacity (given up when memory runs short)
+  ctx->geo_short[0] = ctx->geo_short[1] = false;
   gf_pfree(ctx, ctx->d_K64);
   gf_pfree(ctx, ctx->d_K32);
   gf_sell_free(ctx);
@@ -193,8 +194,15 @@ cudaError_t gf_malloc_retry(gf_ctx* ctx, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
   if (e == cudaErrorMemoryAllocation && !ctx->pool_free.empty()) {
     cudaGetLastError();
-    for (auto& b : ctx->pool_free) cudaFree(b.p);  // give unused blocks back, retry once
+    for (auto& b : ctx->pool_free) cudaFree(b.p);  // give unused blocks back
     ctx->pool_free.clear();
+    e = cudaMalloc(p, bytes);
+  }
+  if (e == cudaErrorMemoryAllocation && ctx->d_geo) {
+    cudaGetLastError();
+    cudaFree(ctx->d_geo);   // scratch of the owner assemblies, which write it anew
+    ctx->d_geo = nullptr;
+    ctx->geo_bytes = 0;
     e = cudaMalloc(p, bytes);
   }
   if (e != cudaSuccess) {
@@ -542,17 +550,20 @@ GF_API gf_status gf_assemble(gf_ctx* ctx, int32_t dtype, int32_t scatter, int32_
   const bool automatic = scatter == GF_SCATTER_AUTO;
   if (automatic)
     scatter = ctx->dim == 2 || engine == GF_ENGINE_TF32_MMA ||
-                      (gf_assemble_node_fits(ctx, dtype) && !b8_small)
+                      (gf_assemble_node_fits(ctx, dtype) && !b8_small && !ctx->geo_short[dtype == GF_F64])
                   ? GF_SCATTER_OWNER
                   : GF_SCATTER_ATOMIC;
   if (scatter == GF_SCATTER_COLOR && ctx->ncolors == 0 &&
       (st = gf_color_build(ctx, nullptr)) != GF_OK)
     return st;
   st = gf_assemble_launch(ctx, dtype, scatter, engine);
-  // no room for Brick8's geometry (320 bytes an element in FP32): atomics do without
+  // no room for Brick8's geometry (320 bytes an element in FP32): atomics do without, and the
+  // pattern's next assemblies don't ask for it again
   if (st == GF_ERR_OOM && automatic && scatter == GF_SCATTER_OWNER &&
-      ctx->elem_type == GF_BRICK8 && engine != GF_ENGINE_TF32_MMA)
+      ctx->elem_type == GF_BRICK8 && engine != GF_ENGINE_TF32_MMA) {
     st = gf_assemble_launch(ctx, dtype, GF_SCATTER_ATOMIC, engine);
+    if (st == GF_OK) ctx->geo_short[dtype == GF_F64] = true;
+  }
   return st;
 }
 
@@ -937,8 +948,8 @@ GF_API gf_status gf_spmv_host(gf_ctx* ctx, int32_t dtype, const double* x, doubl
   void *dx = nullptr, *dy = nullptr;
   gf_status st = GF_OK;
   const size_t es = dtype == GF_F64 ? 8 : 4;
-  if (cudaMalloc(&dx, es * n) != cudaSuccess || cudaMalloc(&dy, es * n) != cudaSuccess) {
-    cudaGetLastError();
+  if (gf_malloc_retry(ctx, &dx, es * n) != cudaSuccess ||
+      gf_malloc_retry(ctx, &dy, es * n) != cudaSuccess) {
     if (dx) cudaFree(dx);
     return gf_fail(ctx, GF_ERR_OOM, "spmv_host buffers");
   }

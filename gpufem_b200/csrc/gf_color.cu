@@ -129,8 +129,7 @@ extern "C" GF_API gf_status gf_mesh_color_device(gf_ctx* ctx, uint64_t seed, int
   k_iota_elems<<<gf_blocks(nelem, kCT), kCT, 0, s>>>(nelem, d_ids);
   size_t tb = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, tb, d_color, d_keys, d_ids, d_perm, nelem, 0, 9, s);
-  if (cudaMalloc(&d_tmp, tb) != cudaSuccess) {
-    cudaGetLastError();
+  if (gf_malloc_retry(ctx, &d_tmp, tb) != cudaSuccess) {
     cleanup();
     return gf_fail(ctx, GF_ERR_OOM, "colour sort scratch");
   }

@@ -243,6 +243,7 @@ struct gf_ctx {
   bool consecutive = false;       // consecutive elements have nodes of like numbers
   void* d_geo = nullptr;          // owner scatter: J^-1, w detJ (E) per (element, Gauss point)
   size_t geo_bytes = 0;
+  bool geo_short[2] = {false, false};  // Brick8 FP32, FP64: no room for it with this pattern
 
   // values
   bool has64 = false, has32 = false;
@@ -309,8 +310,8 @@ gf_status gf_cuda_fail(gf_ctx* ctx, cudaError_t e, const char* where);
     if (e__ != cudaSuccess) return gf_cuda_fail(ctx, e__, name);      \
   } while (0)
 
-// cudaMalloc; when memory is short, the context's unused pool blocks are freed and the
-// allocation is tried once more.
+// cudaMalloc; when memory is short, the context's unused pool blocks, then the owner assemblies'
+// geometry buffer are freed and the allocation is tried again.
 cudaError_t gf_malloc_retry(gf_ctx* ctx, void** p, size_t bytes);
 
 template <typename T>

@@ -197,8 +197,7 @@ gf_status gf_sell_prepare(gf_ctx* ctx, int dtype) {
     ctx->launches++;
     GF_CUDA(ctx, cudaMemsetAsync(wsz + nslice, 0, sizeof(int64_t), s));
     cub::DeviceScan::ExclusiveSum(nullptr, tb, wsz, ctx->d_sell_off, nslice + 1, s);
-    if (cudaMalloc(&tmp, tb) != cudaSuccess) {
-      cudaGetLastError();
+    if (gf_malloc_retry(ctx, &tmp, tb) != cudaSuccess) {
       cudaFree(wsz);
       return gf_fail(ctx, GF_ERR_OOM, "SELL scan scratch");
     }

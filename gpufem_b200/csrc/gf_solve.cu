@@ -812,10 +812,8 @@ gf_status ensure_work(gf_ctx* ctx) {
     if (ctx->d_work) cudaFree(ctx->d_work);
     ctx->d_work = nullptr;
     ctx->work_bytes = 0;
-    if (cudaMalloc(&ctx->d_work, need) != cudaSuccess) {
-      cudaGetLastError();
+    if (gf_malloc_retry(ctx, &ctx->d_work, need) != cudaSuccess)
       return gf_fail(ctx, GF_ERR_OOM, "solver work vectors (%zu bytes)", need);
-    }
     ctx->work_bytes = need;
   }
   if (!ctx->d_u && (st = gf_alloc(ctx, &ctx->d_u, (size_t)ctx->n)) != GF_OK) return st;
@@ -1280,12 +1278,8 @@ gf_status run_fcg(gf_ctx* ctx, const gf_solve_opts* o, int maxit, int check,
   const bool coarse = gf_lp_coarse(ctx);
   if ((st = gf_lp_prepare(ctx)) != GF_OK) return st;
   if (coarse && (st = gf_coarse_prepare(ctx, 0)) != GF_OK) return st;
-  if (!ctx->d_fcg) {
-    if (cudaMalloc(&ctx->d_fcg, sizeof(FcgScalars)) != cudaSuccess) {
-      cudaGetLastError();
-      return gf_fail(ctx, GF_ERR_OOM, "FCG scalars");
-    }
-  }
+  if (!ctx->d_fcg && gf_malloc_retry(ctx, &ctx->d_fcg, sizeof(FcgScalars)) != cudaSuccess)
+    return gf_fail(ctx, GF_ERR_OOM, "FCG scalars");
   FcgScalars* sc = static_cast<FcgScalars*>(ctx->d_fcg);
   FcgScalars hs{};
   double* w = (double*)ctx->d_work;
