@@ -48,9 +48,12 @@ GF_API gf_status gf_create(gf_ctx** out, int32_t device) {
   if (cudaSetDevice(device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess ||
-      cudaEventCreate(&ctx->eva0) != cudaSuccess || cudaEventCreate(&ctx->eva1) != cudaSuccess ||
-      cudaEventCreate(&ctx->evs0) != cudaSuccess || cudaEventCreate(&ctx->evs1) != cudaSuccess ||
-      cudaEventCreate(&ctx->evm) != cudaSuccess) {
+      [&] {
+        for (auto* t : {&ctx->asm_now, &ctx->asm_done, &ctx->call_now, &ctx->call_done})
+          for (auto* e : {&t->e0, &t->em, &t->e1})
+            if (cudaEventCreate(e) != cudaSuccess) return true;
+        return false;
+      }()) {
     cudaGetLastError();
     delete ctx;
     return GF_ERR_CUDA;
@@ -78,11 +81,9 @@ GF_API gf_status gf_destroy(gf_ctx* ctx) {
   gf_pool_clear(ctx);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
-  if (ctx->eva0) cudaEventDestroy(ctx->eva0);
-  if (ctx->eva1) cudaEventDestroy(ctx->eva1);
-  if (ctx->evm) cudaEventDestroy(ctx->evm);
-  if (ctx->evs0) cudaEventDestroy(ctx->evs0);
-  if (ctx->evs1) cudaEventDestroy(ctx->evs1);
+  for (auto* t : {&ctx->asm_now, &ctx->asm_done, &ctx->call_now, &ctx->call_done})
+    for (cudaEvent_t e : {t->e0, t->em, t->e1})
+      if (e) cudaEventDestroy(e);
   if (ctx->ev_dl) cudaEventDestroy(ctx->ev_dl);
   if (ctx->h_adj_stage) cudaFreeHost(ctx->h_adj_stage);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -93,7 +94,7 @@ GF_API gf_status gf_destroy(gf_ctx* ctx) {
 GF_API const char* gf_last_error(const gf_ctx* ctx) { return ctx ? ctx->err.c_str() : "null context"; }
 GF_API double gf_last_device_seconds(const gf_ctx* ctx) {
   if (!ctx) return 0.0;
-  return ctx->timed0 ? gf_elapsed(ctx->timed0, ctx->timed1) : ctx->last_seconds;
+  return ctx->timed ? gf_elapsed(ctx->timed->e0, ctx->timed->e1) : ctx->last_seconds;
 }
 GF_API int64_t gf_kernel_launches(const gf_ctx* ctx) { return ctx ? ctx->launches : 0; }
 
@@ -102,8 +103,9 @@ GF_API gf_status gf_last_assembly_split(const gf_ctx* ctx, double* geometry_seco
   if (!ctx) return GF_ERR_INVALID_ARG;
   double geo = 0.0, scatter = 0.0;
   if (ctx->has_split) {
-    if (ctx->split_owner) geo = gf_elapsed(ctx->eva0, ctx->evm);
-    scatter = gf_elapsed(ctx->split_owner ? ctx->evm : ctx->eva0, ctx->eva1);
+    const gf_ctx::Timer& t = ctx->asm_done;
+    if (ctx->split_owner) geo = gf_elapsed(t.e0, t.em);
+    scatter = gf_elapsed(ctx->split_owner ? t.em : t.e0, t.e1);
   }
   if (geometry_seconds) *geometry_seconds = geo;
   if (scatter_seconds) *scatter_seconds = scatter;

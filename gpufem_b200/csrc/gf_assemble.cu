@@ -356,12 +356,11 @@ gf_status gf_assemble_launch(gf_ctx* ctx, int dtype, int scatter, int engine) {
   if (scatter != GF_SCATTER_OWNER &&
       (st = b20 ? gf_einc_ensure(ctx) : gf_slotmap_ensure(ctx)) != GF_OK)
     return st;
-  ctx->has_split = false;
-  ctx->time_begin(ctx->eva0);
+  cudaEventRecord(ctx->asm_now.e0, ctx->stream);
   if (mma && scatter == GF_SCATTER_OWNER) {
     // tensor cores: every element's Gram matrix to HBM; owner gather: K written once
     st = gf_assemble_tc(ctx, scatter, d_tab, ctx->d_gram, ctx->d_asm_err);
-    cudaEventRecord(ctx->evm, ctx->stream);
+    cudaEventRecord(ctx->asm_now.em, ctx->stream);
     if (st == GF_OK) st = gf_assemble_owner_gram(ctx, ctx->d_gram, ctx->d_K32);
   } else if (scatter == GF_SCATTER_OWNER) {
     // owner-computes: every K entry (padding included) is written exactly once
@@ -375,7 +374,7 @@ gf_status gf_assemble_launch(gf_ctx* ctx, int dtype, int scatter, int engine) {
     st = mma ? gf_assemble_tc(ctx, scatter, d_tab, ctx->d_K32, ctx->d_asm_err)
              : launch_dispatch<float>(ctx, scatter, d_tab, ctx->d_K32);
   }
-  cudaEventRecord(ctx->eva1, ctx->stream);
+  cudaEventRecord(ctx->asm_now.e1, ctx->stream);
   cudaError_t e = cudaStreamSynchronize(ctx->stream);
   if (st != GF_OK) return st;
   if (e != cudaSuccess) return gf_cuda_fail(ctx, e, "assembly");
@@ -385,7 +384,7 @@ gf_status gf_assemble_launch(gf_ctx* ctx, int dtype, int scatter, int engine) {
     if (herr)
       return gf_fail(ctx, GF_ERR_CUDA, "tensor-core assembly: an MMA completion wait timed out");
   }
-  ctx->time_end(ctx->eva0, ctx->eva1);
+  ctx->time_end(ctx->asm_now, ctx->asm_done);
   ctx->has_split = true;
   ctx->split_owner = scatter == GF_SCATTER_OWNER;
   if (dtype == GF_F64) { ctx->has64 = true; ctx->kver64++; } else { ctx->has32 = true; ctx->kver32++; }

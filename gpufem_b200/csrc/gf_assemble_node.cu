@@ -618,7 +618,7 @@ gf_status launch_geometry(gf_ctx* ctx) {
   k_geometry<ET, T, NG1, IL><<<gf_blocks(ctx->nelem, kGT), kGT, 0, ctx->stream>>>(
       ctx->nelem, ctx->d_conn, ctx->d_coords64, Eel, (T*)ctx->d_geo);
   GF_LAUNCH_CHECK(ctx, "k_geometry");
-  cudaEventRecord(ctx->evm, ctx->stream);
+  cudaEventRecord(ctx->asm_now.em, ctx->stream);
   return GF_OK;
 }
 

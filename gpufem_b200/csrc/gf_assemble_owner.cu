@@ -587,7 +587,7 @@ gf_status launch_owner(gf_ctx* ctx, TC* K, const AsmTables* d_tab) {
         ctx->nelem, ngp, EB, ctx->d_conn, ctx->d_coords64, d_tab, geo);
   }
   GF_LAUNCH_CHECK(ctx, "k_elem_geometry");
-  cudaEventRecord(ctx->evm, ctx->stream);
+  cudaEventRecord(ctx->asm_now.em, ctx->stream);
   // largest node block (at most 128: the owning node index is a byte) whose tile keeps
   // three CTAs per SM; small meshes take smaller blocks so that every SM gets two CTAs
   // (Q4 64^2, 4,225 nodes: 25 us with 33 CTAs of 128 nodes, 20 us with 66 of 64; on

@@ -165,27 +165,24 @@ struct gf_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  cudaEvent_t eva0 = nullptr, eva1 = nullptr;  // around the last assembly
-  cudaEvent_t evm = nullptr;            // between the two kernels of an owner assembly
-  cudaEvent_t evs0 = nullptr, evs1 = nullptr;  // around the last gf_spmv or gf_lp_apply
-  bool has_split = false, split_owner = false;  // eva0, eva1 (and evm) hold an assembly
+  // Events of a short timed call, before (0), between the two kernels of an owner assembly (m) and
+  // after (1); `done` ones hold the last call that succeeded, the others are recorded meanwhile.
+  struct Timer { cudaEvent_t e0 = nullptr, em = nullptr, e1 = nullptr; };
+  Timer asm_now, asm_done;      // assemblies
+  Timer call_now, call_done;    // gf_spmv and gf_lp_apply
+  bool has_split = false, split_owner = false;  // asm_done holds an assembly, one by owners
   std::string err;
   // Device time of the last timed call: last_seconds, or between two events whose elapsed time is
   // taken when asked for (each such query costs a short call 3 us).
   double last_seconds = 0.0;
-  cudaEvent_t timed0 = nullptr, timed1 = nullptr;
+  const Timer* timed = nullptr;
   void set_seconds(double s) {
     last_seconds = s;
-    timed0 = timed1 = nullptr;
+    timed = nullptr;
   }
-  // Around a short timed call: its events hold nothing until it has succeeded.
-  void time_begin(cudaEvent_t e0) {
-    if (timed0 == e0) set_seconds(0.0);
-    cudaEventRecord(e0, stream);
-  }
-  void time_end(cudaEvent_t e0, cudaEvent_t e1) {
-    timed0 = e0;
-    timed1 = e1;
+  void time_end(Timer& now, Timer& done) {   // the call has succeeded
+    std::swap(now, done);
+    timed = &done;
   }
   int64_t launches = 0;
   int sm_count = 148;

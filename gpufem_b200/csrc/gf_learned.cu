@@ -1139,13 +1139,13 @@ GF_API gf_status gf_lp_apply(gf_ctx* ctx, const float* r, float* z) {
   gf_status st = gf_lp_prepare(ctx);
   if (st != GF_OK) return st;
   LpState* s = ctx->lp;
-  ctx->time_begin(ctx->evs0);
+  cudaEventRecord(ctx->call_now.e0, ctx->stream);
   lp_forward(ctx, r, false);
   k_lp_output<float><<<gf_blocks(s->n, kLT), kLT, 0, ctx->stream>>>(s->n, s->rho, s->y, s->sc, z);
   GF_LAUNCH_CHECK(ctx, "k_lp_output");
-  cudaEventRecord(ctx->evs1, ctx->stream);
+  cudaEventRecord(ctx->call_now.e1, ctx->stream);
   if ((st = lp_check_err(ctx)) != GF_OK) return st;   // waits for the stream
-  ctx->time_end(ctx->evs0, ctx->evs1);
+  ctx->time_end(ctx->call_now, ctx->call_done);
   return GF_OK;
 }
 

@@ -651,7 +651,7 @@ gf_status gf_spmv_launch(gf_ctx* ctx, int dtype, const void* x, void* y) {
   // 2-D node blocks read x in pairs (one 8- or 16-byte load per neighbour node)
   if (L.bdim == 2 && ((uintptr_t)x % (dtype == GF_F64 ? 16 : 8)) != 0)
     return gf_fail(ctx, GF_ERR_INVALID_ARG, "x must be aligned to two entries");
-  ctx->time_begin(ctx->evs0);
+  cudaEventRecord(ctx->call_now.e0, ctx->stream);
   if (dtype == GF_F64)
     GF_ROWS_LAUNCH(ctx, ctx->stream, L, (k_spmv<Walk, double, double, double>),
                    (const double*)val, (const double*)x, (double*)y);
@@ -659,9 +659,9 @@ gf_status gf_spmv_launch(gf_ctx* ctx, int dtype, const void* x, void* y) {
     GF_ROWS_LAUNCH(ctx, ctx->stream, L, (k_spmv<Walk, float, float, float>),
                    (const float*)val, (const float*)x, (float*)y);
   GF_LAUNCH_CHECK(ctx, "k_spmv");
-  cudaEventRecord(ctx->evs1, ctx->stream);
-  GF_CUDA(ctx, cudaEventSynchronize(ctx->evs1));
-  ctx->time_end(ctx->evs0, ctx->evs1);
+  cudaEventRecord(ctx->call_now.e1, ctx->stream);
+  GF_CUDA(ctx, cudaEventSynchronize(ctx->call_now.e1));
+  ctx->time_end(ctx->call_now, ctx->call_done);
   return GF_OK;
 }
 
