@@ -12,9 +12,9 @@
 // range of nodes to a CTA, and is gathered from there.  An iteration exchanges three things: p.q,
 // then (r.z, r.r), then the new p.  With copies they are asynchronous stores that complete on a
 // barrier of the CTA they go to, which waits for their bytes alone; a buffer is written again only
-// after an answer that its reader sends when it is done with it.  Waits are bounded; a CTA that
-// gives up leaves the iteration as a whole, and the others follow.  Without copies there is a
-// cluster barrier after each.  Each CTA adds all parts of a sum in the same order, so a solve is
+// after an answer that its reader sends when it is done with it.  Waits are bounded in time; a CTA
+// that gives up tells the others and leaves the iteration as a whole, and the others follow when
+// their own waits run out.  Without copies there is a cluster barrier after each.  Each CTA adds all parts of a sum in the same order, so a solve is
 // reproducible.
 //
 // Microseconds per iteration (FP64 Jacobi-PCG; the same with cluster barriers; gathering from the
@@ -139,19 +139,25 @@ __device__ __forceinline__ void st_async_node(uint32_t a, const float (&v)[DIM],
 __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Waits for the phase of parity `parity`; false if it does not come.
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-  for (int k = 0; k < 20000; ++k) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok)
-                 : "r"(bar), "r"(parity)
-                 : "memory");
-    if (ok) return true;
-  }
-  return false;
+__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {   // for a short while
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\t"
+               "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+               "selp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok)
+               : "r"(bar), "r"(parity)
+               : "memory");
+  return ok;
+}
+// Waits for the phase of parity `parity`, `limit` clocks at most; false if it does not come (a
+// negative limit: at once).
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, long long limit) {
+  if (limit < 0) return false;
+  if (bar_try(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!bar_try(bar, parity))
+    if (clock64() - t0 >= limit) return false;
+  return true;
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -167,7 +173,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 template <int N, bool ASYNC>
 __device__ __forceinline__ bool cluster_sum(double (&v)[N], int S, double* sh, double* part,
                                             uint32_t part_addr, uint32_t bar, uint32_t parity,
-                                            bool& late) {
+                                            long long limit, bool& late) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp < S) {
 #pragma unroll
@@ -196,7 +202,7 @@ __device__ __forceinline__ bool cluster_sum(double (&v)[N], int S, double* sh, d
     }
   }
   if constexpr (ASYNC)
-    late = !bar_wait(bar, parity);
+    late = !bar_wait(bar, parity, limit);
   else
     cluster_sync();
 #pragma unroll
@@ -212,6 +218,7 @@ __device__ __forceinline__ bool cluster_sum(double (&v)[N], int S, double* sh, d
 struct ClusterArgs {
   int nnodes, S, H, iters, jacobi;   // S slices per CTA, H warps per slice
   double eps;
+  long long limit;                   // of a wait for another CTA, in clocks
   const int32_t* __restrict__ perm;
   const int32_t* __restrict__ width;
   const int64_t* __restrict__ off;
@@ -242,6 +249,7 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
   // directions: [per][DIM] of this CTA's nodes, or [nnodes][DIM] where copies are kept
   uint64_t* bars = reinterpret_cast<uint64_t*>(sh + 64);     // p.q; r.z and r.r; directions
   uint32_t* count = reinterpret_cast<uint32_t*>(bars + 3);   // nodes whose directions come here
+  uint32_t* gave_up = count + 1;                             // a CTA's wait has run out
   V* sp = reinterpret_cast<V*>(bars + 4);
   uint32_t* smask = reinterpret_cast<uint32_t*>(                // [per] CTAs that read a node's
       reinterpret_cast<unsigned char*>(sp) + (sizeof(V) * DIM * A.nnodes + 15) / 16 * 16);
@@ -267,7 +275,7 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
   if constexpr (COPY) {
     for (int i = threadIdx.x; i < per; i += blockDim.x) smask[i] = 0;
     if (threadIdx.x == 0) {
-      *count = 0;
+      *count = *gave_up = 0;
 #pragma unroll
       for (int k = 0; k < 3; ++k)
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8 * k) : "memory");
@@ -347,7 +355,7 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
         two[0] += (double)rv[c] * (double)pv[c];
         two[1] += (double)rv[c] * (double)rv[c];
       }
-    cluster_sum<2, false>(two, S, sh, partB, pb, 0, 0, late);
+    cluster_sum<2, false>(two, S, sh, partB, pb, 0, 0, 0, late);
     rz = two[0];
     rr = two[1];
     tol2 = A.eps * A.eps * rr;
@@ -357,7 +365,7 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
   if (!COPY) cluster_sync();
   for (int step = 0; step < A.iters; ++step) {
     const uint32_t parity = step & 1;
-    if (COPY) late = !bar_wait(bar + 16, parity);
+    if (COPY) late = !bar_wait(bar + 16, parity, A.limit);
     V q[DIM];
 #pragma unroll
     for (int c = 0; c < DIM; ++c) q[c] = V(0);
@@ -387,7 +395,7 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
     double sum[1] = {0.0};
 #pragma unroll
     for (int c = 0; c < DIM; ++c) sum[0] += (double)pv[c] * (double)q[c];
-    if (cluster_sum<1, COPY>(sum, S, sh, partA, pa, bar, parity, late)) {
+    if (cluster_sum<1, COPY>(sum, S, sh, partA, pa, bar, parity, A.limit, late)) {
       done = 4;
       break;
     }
@@ -407,7 +415,7 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
         two[1] += (double)rv[c] * (double)rv[c];
       }
     }
-    if (cluster_sum<2, COPY>(two, S, sh, partB, pb, bar + 8, parity, late)) {
+    if (cluster_sum<2, COPY>(two, S, sh, partB, pb, bar + 8, parity, A.limit, late)) {
       done = 4;
       break;
     }
@@ -432,9 +440,16 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
     publish(pv);
     if (!COPY) cluster_sync();
   }
-  if (done == 4)
-    for (int k = 0; k < 100; ++k) __nanosleep(1000);   // what is under way arrives
+  if (done == 4 && threadIdx.x < kCluster)   // to every CTA: CTA 0 may have ended as usual
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_rank(bar + 28, threadIdx.x)), "r"(1u) : "memory");
   cluster_sync();   // no CTA leaves while another may still write to it
+  if (COPY && *gave_up) {
+    // nothing is sent any more, but stores to a CTA that gave up may be under way: 0.1 ms
+    const long long t0 = clock64();
+    for (int k = 0; k < 100000 && clock64() - t0 < 200000; ++k) __nanosleep(200);
+    done = 4;
+    cluster_sync();
+  }
   if (on)
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
@@ -458,7 +473,7 @@ k_pcg_cluster(ClusterArgs A, const V* __restrict__ val, const V* __restrict__ di
 template <int DIM, typename V, bool COPY>
 gf_status run_cluster_as(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V* p, double eps,
                          int iters, int* ran) {
-  *ran = 0;
+  *ran = kPcgNotRun;
   if (iters < 1) return GF_OK;
   const int nslice = (ctx->nnodes + 31) / 32;
   const int S = (nslice + kCluster - 1) / kCluster;
@@ -472,8 +487,8 @@ gf_status run_cluster_as(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V
   auto kern = k_pcg_cluster<DIM, V, COPY>;
   GF_CUDA(ctx, gf_smem_attr(kern, sm));
   GF_CUDA(ctx, gf_func_attr((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  ClusterArgs A{ctx->nnodes, S, H, iters, dinv != nullptr, eps, ctx->d_sell_perm, ctx->d_sell_w,
-                ctx->d_sell_off, ctx->d_sell_col, ctx->d_scal};
+  ClusterArgs A{ctx->nnodes, S, H, iters, dinv != nullptr, eps, ctx->pcg_wait, ctx->d_sell_perm,
+                ctx->d_sell_w, ctx->d_sell_off, ctx->d_sell_col, ctx->d_scal};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = kCluster;
@@ -495,7 +510,7 @@ gf_status run_cluster_as(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V
   GF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (static_cast<const SolveScalars*>(ctx->h_pinned)->done == 4)
     return gf_fail(ctx, GF_ERR_CUDA, "PCG on a cluster: a wait for another CTA timed out");
-  *ran = 1;
+  *ran = kPcgRan;
   return GF_OK;
 }
 
@@ -504,27 +519,32 @@ template <int DIM, typename V>
 gf_status run_cluster(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V* p, double eps, int iters,
                       int* ran) {
   const gf_status st = run_cluster_as<DIM, V, true>(ctx, val, dinv, x, r, p, eps, iters, ran);
-  if (st != GF_OK || *ran) return st;
+  if (st != GF_OK || *ran != kPcgNotRun) return st;
   return run_cluster_as<DIM, V, false>(ctx, val, dinv, x, r, p, eps, iters, ran);
 }
 
 }  // namespace
 
 // Runs up to `iters` iterations of the (P)CG to the tolerance eps whose state is in x, r, p and the
-// context's scalars
-// (iter, rr, rzn, done updated and read back to the pinned copy).  *ran = 0: the system is not
-// one for this kernel, and nothing was done.  dinv = null: no preconditioner.
+// context's scalars (iter, rr, rzn, done updated and read back to the pinned copy).  *ran =
+// kPcgNotRun: the system is not one for this kernel, and nothing was done.  dinv = null: no
+// preconditioner.
 gf_status gf_pcg_cluster(gf_ctx* ctx, const double* val, const double* dinv, double* x, double* r,
                          double* p, double eps, int iters, int* ran) {
-  *ran = 0;
+  *ran = kPcgNotRun;
   if (ctx->sell_bdim == 2) return run_cluster<2, double>(ctx, val, dinv, x, r, p, eps, iters, ran);
   if (ctx->sell_bdim == 3) return run_cluster<3, double>(ctx, val, dinv, x, r, p, eps, iters, ran);
   return GF_OK;
 }
 gf_status gf_pcg_cluster(gf_ctx* ctx, const float* val, const float* dinv, float* x, float* r,
                          float* p, double eps, int iters, int* ran) {
-  *ran = 0;
+  *ran = kPcgNotRun;
   if (ctx->sell_bdim == 2) return run_cluster<2, float>(ctx, val, dinv, x, r, p, eps, iters, ran);
   if (ctx->sell_bdim == 3) return run_cluster<3, float>(ctx, val, dinv, x, r, p, eps, iters, ran);
   return GF_OK;
+}
+
+// For the tests only: the limit of a wait in clocks (negative: every wait runs out).
+extern "C" __attribute__((visibility("default"))) void gftest_pcg_wait(gf_ctx* ctx, long long clocks) {
+  ctx->pcg_wait = clocks;
 }

@@ -741,20 +741,24 @@ gf_status run_cg(gf_ctx* ctx, MatLayout L, const TK* val, const V* b, CgVecs vv,
   V *x = (V*)vv.x, *r = (V*)vv.r, *z = (V*)vv.z, *p = (V*)vv.p, *q = (V*)vv.q;
   const V* dinv = precond ? (const V*)vv.dinv : nullptr;
   V* zz = precond ? z : r;  // without a preconditioner z aliases r
-  GF_CUDA(ctx, cudaMemsetAsync(sc, 0, sizeof(SolveScalars), s));
-  k_cg_init<V><<<red_grid(ctx, n), kT, 0, s>>>(n, b, dinv, x, r, zz, p, sc);
-  GF_LAUNCH_CHECK(ctx, "k_cg_init");
-  k_cg_init_fin<<<1, 1, 0, s>>>(sc, eps, maxit);
-  GF_LAUNCH_CHECK(ctx, "k_cg_init_fin");
+  auto begin = [&]() -> gf_status {
+    GF_CUDA(ctx, cudaMemsetAsync(sc, 0, sizeof(SolveScalars), s));
+    k_cg_init<V><<<red_grid(ctx, n), kT, 0, s>>>(n, b, dinv, x, r, zz, p, sc);
+    GF_LAUNCH_CHECK(ctx, "k_cg_init");
+    k_cg_init_fin<<<1, 1, 0, s>>>(sc, eps, maxit);
+    GF_LAUNCH_CHECK(ctx, "k_cg_init_fin");
+    return GF_OK;
+  };
+  gf_status st = begin();
+  if (st != GF_OK) return st;
   SolveScalars* hs = (SolveScalars*)ctx->h_pinned;
   // small systems: every iteration in one kernel (with a time limit, a launch per check_every
   // iterations)
   for (;;) {
-    int ran = 0;
-    gf_status st = gf_pcg_cluster(ctx, val, dinv, x, r, p, eps,
-                                  max_seconds > 0.0 ? check_every : maxit, &ran);
+    int ran = kPcgNotRun;
+    st = gf_pcg_cluster(ctx, val, dinv, x, r, p, eps, max_seconds > 0.0 ? check_every : maxit, &ran);
     if (st != GF_OK) return st;
-    if (!ran) break;
+    if (ran != kPcgRan) break;
     if (!hs->done && max_seconds > 0.0 &&
         std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() <= max_seconds)
       continue;
@@ -781,7 +785,6 @@ gf_status run_cg(gf_ctx* ctx, MatLayout L, const TK* val, const V* b, CgVecs vv,
     cudaGraphDestroy(graph);
     return gf_cuda_fail(ctx, ce, "graph instantiate");
   }
-  gf_status st = GF_OK;
   for (;;) {
     ce = cudaGraphLaunch(exec, s);
     if (ce != cudaSuccess) { st = gf_cuda_fail(ctx, ce, "graph launch"); break; }
