@@ -185,7 +185,7 @@ struct gf_ctx {
     timed = &done;
   }
   int64_t launches = 0;
-  long long pcg_wait = 2000000000;  // clocks that a CTA of k_pcg_cluster waits for another: 1 s
+  int pcg_late = -1;  // gftest_pcg_late
   int sm_count = 148;
 
   // mesh
@@ -413,7 +413,7 @@ gf_status gf_matvec_f32(gf_ctx* ctx, const float* x, const float* scale, float* 
 gf_status gf_solve_run(gf_ctx* ctx, const gf_solve_opts* o, gf_solve_info* info);
 void gf_solver_free(gf_ctx* ctx);
 // (P)CG in one kernel (gf_pcg_cluster.cu)
-constexpr int kPcgNotRun = 0, kPcgRan = 1;
+constexpr int kPcgNotRun = 0, kPcgRan = 1, kPcgGaveUp = 2;
 gf_status gf_pcg_cluster(gf_ctx* ctx, const double* val, const double* dinv, double* x, double* r,
                          double* p, double eps, int iters, int* ran);
 gf_status gf_pcg_cluster(gf_ctx* ctx, const float* val, const float* dinv, float* x, float* r,

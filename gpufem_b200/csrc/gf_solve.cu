@@ -758,6 +758,7 @@ gf_status run_cg(gf_ctx* ctx, MatLayout L, const TK* val, const V* b, CgVecs vv,
     int ran = kPcgNotRun;
     st = gf_pcg_cluster(ctx, val, dinv, x, r, p, eps, max_seconds > 0.0 ? check_every : maxit, &ran);
     if (st != GF_OK) return st;
+    if (ran == kPcgGaveUp && (st = begin()) != GF_OK) return st;   // from the start, as a graph
     if (ran != kPcgRan) break;
     if (!hs->done && max_seconds > 0.0 &&
         std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count() <= max_seconds)
