@@ -11,7 +11,8 @@ L2 flushed between steps; the colour, atomic and TF32 tensor-core variants are t
 beside it.  `e2e` = the same metric through the public C-ABI from pinned host buffers:
 mesh upload, pattern, assembly and download of the ELL matrix, every step.  For N > 1 each
 rank assembles its own replica of the workload (weak scaling; the assembly needs
-no exchange) and the time is the max over ranks.
+no exchange) and the time is the max over ranks.  The line summarises the solver and learned
+studies; they go to stderr in full, before it.
 """
 from __future__ import annotations
 
@@ -675,6 +676,30 @@ def run_sharded_arm(args):
     dist.destroy_process_group()
 
 
+def short_line(line):
+    """The line for stdout, short enough to be kept whole by a log's tail (3,000 characters), and the
+    blocks that it only summarises."""
+    def brief(d):
+        return {k: float(f"{v:.4g}") for k, v in d.items() if isinstance(v, (int, float))}
+
+    def study(d):
+        d = d.get("solve", d)
+        return {"target_rel_error": d["target_rel_error"],
+                "total_seconds": brief({k: v["total_seconds"] for k, v in d.items()
+                                        if isinstance(v, dict) and "total_seconds" in v})}
+
+    summaries = {
+        "solve": study, "brick20_64": study, "learned": lambda d: brief(d["summary"]),
+        "roofline_assembly": lambda d: brief({k: d[k] for k in ("achieved", "frac")}),
+        "roofline_spmv": lambda d: brief({k: d[k] for k in ("achieved", "frac")}),
+        "scatter_variants": lambda d: brief({k: v["value"] for k, v in d.items()}),
+    }
+    details = {k: line[k] for k in summaries if line.get(k)}
+    short = {k: v for k, v in line.items() if k not in summaries}
+    short.update({k: summaries[k](d) for k, d in details.items()})
+    return short, details
+
+
 def run_gpu_arm(args):
     import torch
     rank, world, local = dist_info()
@@ -945,6 +970,8 @@ def run_gpu_arm(args):
             "learned": learned,
             "cpu_baseline": cpu_baseline,
         }
+        line, details = short_line(line)
+        print(json.dumps({"details": details}), file=sys.stderr, flush=True)
         print(json.dumps(line), flush=True)
     ctx.close()
     if world > 1:
