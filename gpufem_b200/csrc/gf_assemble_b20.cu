@@ -418,8 +418,15 @@ gf_status launch_b20(gf_ctx* ctx, const AsmTables* d_tab, T* K) {
   // nodes do not fill the lines in order, most of it is fetched for nothing, and twice: FP32 56^3
   // with the nodes shuffled in runs of 128, 16, 1 3128, 7372, 13869 against 2544, 4303, 9451, rows
   // of 8 elements (8 x 8 x 3200) 2964 against 2412, of 16 2521 against 2451, of 52 1819 against 2047.
-  const bool ahead = ctx->consecutive && (int64_t)ctx->n * ctx->W * (int64_t)sizeof(T) > 1500000000;
-  kern<<<std::min(groups, ctx->sm_count * 2), L::THREADS, L::bytes, ctx->stream>>>(
+  const int64_t kbytes = (int64_t)ctx->n * ctx->W * (int64_t)sizeof(T);
+  const bool ahead = ctx->consecutive && kbytes > 1500000000;
+  // CTAs that stay for several groups drift apart, and with them the elements in flight, whose lines
+  // L2 has to hold at once.  An ordered mesh's are few, and the loads ahead pay: FP32 28^3 249 us,
+  // 263 with a CTA per group, 40^3 702, 665, 56^3 1932, 1976; FP64 36^3 932, 1085.  Shuffled in runs
+  // of 16 nodes: FP32 28^3 351, 344; 32^3 582, 486; 36^3 941, 739; 56^3 4325, 3016 (N = 1: 36^3 2107,
+  // 1850; elements in runs of 16: 651, 690); FP64 36^3 1392, 1377.
+  const bool stay = sizeof(T) == 8 || !ctx->shuffled || kbytes <= 300000000;
+  kern<<<stay ? std::min(groups, ctx->sm_count * 2) : groups, L::THREADS, L::bytes, ctx->stream>>>(
       ctx->nelem, ctx->n, ctx->d_conn, ctx->d_coords64, Eel, ctx->d_einc, ctx->d_inc_slot, d_tab,
       T(ctx->lam1), T(ctx->mu1), ahead, K);
   GF_LAUNCH_CHECK(ctx, "k_assemble_b20");

@@ -238,7 +238,8 @@ struct gf_ctx {
   int32_t* d_einc = nullptr;      // [nelem][nen] incidence of each element node (Brick20 atomic)
   int maxval = 0;                 // max elements sharing one node
   bool scattered = false;         // consecutive nodes lie in elements of unlike numbers
-  bool consecutive = false;       // consecutive elements have nodes of like numbers
+  bool consecutive = false;       // consecutive elements have nodes of like numbers,
+  bool shuffled = false;          // or of unlike ones (neither: short rows)
   void* d_geo = nullptr;          // owner scatter: J^-1, w detJ (E) per (element, Gauss point)
   size_t geo_bytes = 0;
   bool geo_short[2] = {false, false};  // Brick8 FP32, FP64: no room for it with this pattern

@@ -784,6 +784,7 @@ gf_status gf_pattern_build(gf_ctx* ctx) {
   // lexicographic meshes of long rows 0.043, rows of 16 or 8 elements 0.047 or 0.051, runs of
   // shuffled nodes or elements 0.057 and more
   ctx->consecutive = h_end[3] <= 0.046 * h_end[4];
+  ctx->shuffled = h_end[3] > 0.056 * h_end[4];
   ctx->d_inc_off = d_inc_off;  // ownership moves to the context
   ctx->d_inc = d_inc;
   d_inc_off = nullptr;
