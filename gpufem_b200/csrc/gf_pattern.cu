@@ -576,28 +576,38 @@ __global__ void k_incidence_finish(int nnodes, int nen, const int32_t* __restric
 
 // Samples of the mesh's numbering, spread evenly over it: for kLocalityWarps runs of 32
 // consecutive nodes, out[0] += the distinct groups of eight consecutive elements among their
-// first elements, out[1] += nodes; for as many runs of 32 consecutive elements, out[2] += the
+// first elements, out[1] += nodes, and out[4] += the distinct blocks of 32 ids among their
+// neighbours a quarter down their lists; for as many runs of 32 consecutive elements, out[2] += the
 // distinct blocks of 256 ids among their first nodes, out[3] += elements.
 constexpr int kLocalityWarps = 256;
 __global__ void __launch_bounds__(128)
 k_locality(int nnodes, int nelem, int nen, const int32_t* __restrict__ conn,
            const int32_t* __restrict__ inc_off, const int32_t* __restrict__ inc,
+           const int32_t* __restrict__ adj_off, const int32_t* __restrict__ adj,
            int32_t* __restrict__ out) {
+  __shared__ int sum[5];   // a block's counts, so that few atomics meet in one place
+  if (threadIdx.x < 5) sum[threadIdx.x] = 0;
+  __syncthreads();
   const int w = (blockIdx.x * 128 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   auto start = [&](int count) { return (int)((int64_t)max(0, count - 32) * w / (kLocalityWarps - 1)); };
-  auto add = [&](bool on, int key, int32_t* to) {
+  auto add = [&](bool on, int key, int distinct, int count) {
     const unsigned same = __match_any_sync(0xffffffffu, on ? key : -1);
     const unsigned firsts = __ballot_sync(0xffffffffu, on && __ffs(same) - 1 == lane);
     const unsigned all = __ballot_sync(0xffffffffu, on);
     if (lane == 0) {
-      atomicAdd(to, __popc(firsts));
-      atomicAdd(to + 1, __popc(all));
+      atomicAdd(&sum[distinct], __popc(firsts));
+      if (count) atomicAdd(&sum[count], __popc(all));
     }
   };
   const int a = start(nnodes) + lane, e = start(nelem) + lane;
   const bool node = a < nnodes && inc_off[a + 1] > inc_off[a], elem = e < nelem;
-  add(node, node ? inc[inc_off[a]] >> 3 : 0, out);
-  add(elem, elem ? conn[(int64_t)e * nen] >> 8 : 0, out + 2);
+  const int first = node ? inc[inc_off[a]] >> 3 : 0, corner = elem ? conn[(int64_t)e * nen] >> 8 : 0;
+  const int near = node ? adj[adj_off[a] + (adj_off[a + 1] - adj_off[a]) / 4] >> 5 : 0;
+  add(node, first, 0, 1);
+  add(elem, corner, 2, 3);
+  add(node, near, 4, 0);
+  __syncthreads();
+  if (threadIdx.x < 5) atomicAdd(out + threadIdx.x, sum[threadIdx.x]);
 }
 
 }  // namespace
@@ -636,12 +646,12 @@ gf_status gf_pattern_build(gf_ctx* ctx) {
   GF_TRY(gf_palloc(ctx, &d_fill, (size_t)nnodes + 1));
   GF_TRY(gf_palloc(ctx, &d_inc, (size_t)total));
   GF_TRY(gf_palloc(ctx, &d_nadj, (size_t)nnodes + 1));
-  GF_TRY(gf_palloc(ctx, &d_err, 5));   // error, then k_locality's counts
+  GF_TRY(gf_palloc(ctx, &d_err, 6));   // error, then k_locality's counts
   GF_TRY(gf_palloc(ctx, &d_max, 2));
   GF_TRY(gf_palloc(ctx, &ctx->d_adj_off, (size_t)nnodes + 1));
   GF_TRYC(cudaMemsetAsync(d_cnt, 0, sizeof(int32_t) * (nnodes + 1), s));
   GF_TRYC(cudaMemsetAsync(d_nadj, 0, sizeof(int32_t) * (nnodes + 1), s));
-  GF_TRYC(cudaMemsetAsync(d_err, 0, 5 * sizeof(int32_t), s));
+  GF_TRYC(cudaMemsetAsync(d_err, 0, 6 * sizeof(int32_t), s));
 
   cub::DeviceScan::ExclusiveSum(nullptr, b1, d_cnt, d_inc_off, nnodes + 1, s);
   cub::DeviceReduce::Max(nullptr, b2, d_nadj, d_max, nnodes, s);
@@ -768,10 +778,10 @@ gf_status gf_pattern_build(gf_ctx* ctx) {
     ctx->launches++;
   }
   k_locality<<<kLocalityWarps / 4, 128, 0, s>>>(nnodes, nelem, nen, ctx->d_conn, d_inc_off, d_inc,
-                                               d_err + 1);
+                                               ctx->d_adj_off, ctx->d_adj, d_err + 1);
   ctx->launches++;
   GF_TRYC(cudaGetLastError());
-  int32_t h_end[5] = {0, 0, 0, 0, 0};
+  int32_t h_end[6] = {0, 0, 0, 0, 0, 0};
   GF_TRYC(cudaMemcpyAsync(h_end, d_err, sizeof(h_end), cudaMemcpyDeviceToHost, s));
   GF_TRYC(cudaStreamSynchronize(s));
   if (h_end[0]) {
@@ -785,6 +795,7 @@ gf_status gf_pattern_build(gf_ctx* ctx) {
   // shuffled nodes or elements 0.057 and more
   ctx->consecutive = h_end[3] <= 0.046 * h_end[4];
   ctx->shuffled = h_end[3] > 0.056 * h_end[4];
+  ctx->gather = h_end[5] / (float)std::max(1, h_end[2]);
   ctx->d_inc_off = d_inc_off;  // ownership moves to the context
   ctx->d_inc = d_inc;
   d_inc_off = nullptr;

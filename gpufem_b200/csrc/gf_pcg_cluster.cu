@@ -482,6 +482,13 @@ gf_status run_cluster_as(gf_ctx* ctx, const V* val, const V* dinv, V* x, V* r, V
   const int nslice = (ctx->nnodes + 31) / 32;
   const int S = (nslice + kCluster - 1) / kCluster;
   if (S > kThreadsMax / 32) return GF_OK;
+  // Gathers from other CTAs: about 3 ns (2-D: 2 ns) for each separate piece that a warp's lanes
+  // read.  Us an iteration by pieces per CTA, and of the three-kernel loop: FP32 Brick8 13^3 965
+  // 10.5, 2014 13.1, 3093 17.0, 9187 37.1, loop 13.5; FP64 Brick8 10^3 480 9.3, 2202 14.7, 3047
+  // 15.8, loop 14.9; FP32 Q4 124^2 549 5.0, 2680 9.0, 3870 11.5, 7662 24.4, loop 11.0; FP64 Q4 85^2
+  // 265 4.3, 2767 8.7, 3458 11.7, loop 10.7 (ordered meshes first, random ones last).
+  const double pieces = (double)S * 32 * (ctx->W / DIM) * (DIM == 2 ? 1 : 3) * ctx->gather;
+  if (!COPY && pieces > (DIM == 2 ? 3300 : 2100)) return GF_OK;
   // a CTA's slices at the widest row
   const size_t slices = (size_t)S * 32 * (ctx->W / DIM) * (DIM * DIM * sizeof(V) + 4);
   int H = 1;
