@@ -53,7 +53,8 @@ struct Coarse {
   int ntiles = 0;                 // nt (nt + 1) / 2 tiles (I <= J) of the symmetric inverse
   int2* tile_ij = nullptr;        // [ntiles] (I, J)
   double* ainv = nullptr;         // [ntiles][64][64], zero beyond nc
-  int nblk = 0;                   // blocks of the fused update
+  bool fused = true;              // the update of x and r and the restriction in one kernel
+  int nblk = 0;                   // its blocks, or those of the restriction
   int4* blk = nullptr;            // [nblk] aggregate, first node, end, row of rc + 256 blocks
   int parts = 1;                  // rows of rc that hold the sums of an aggregate of mean size
   uint8_t* shares = nullptr;      // [64 nt] rows of rc that an entry sums, if any more than parts
@@ -977,6 +978,18 @@ k_prolong(int n, const int32_t* __restrict__ agg, const double* __restrict__ x,
 // so z is never stored: r.D^-1 r comes with the x/r update, rc.zc with the coarse
 // product.
 
+// alpha = rz / p.q; false when the solve is over, or breaks down with p.q
+__device__ __forceinline__ bool tl_alpha(SolveScalars* sc, double& alpha) {
+  if (sc->done) return false;
+  const double pq = sc->pq;
+  if (!(pq > 0.0) || !isfinite(pq)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) sc->done = 2;
+    return false;
+  }
+  alpha = sc->rz / pq;
+  return true;
+}
+
 // INIT: x = 0, r = scale * b.  Else: alpha = rz / p.q, x += alpha p, r -= alpha q.
 // Accumulates rr = r.r and rzn += r.D^-1 r (in FP64 whatever the vector type V), and restricts
 // r: every node is in one aggregate, so a block takes a share of an aggregate's node list
@@ -992,8 +1005,18 @@ k_prolong(int n, const int32_t* __restrict__ agg, const double* __restrict__ x,
 // aggregate.  With the same number for all, the iteration waited for the largest: Brick8 40^3,
 // 64^3 with 73% of the nodes in one box 170, 802 us -> 58, 171 (uniform 43, 129); coordinates
 // cubed 92, 241 -> 51, 134; Q4 200^2 cubed 50 -> 26 (uniform 18.5).
+// FUSED = false: only the restriction of r.  On a scattered numbering an aggregate's nodes lie at
+// random addresses, and a node's 16 to 24 bytes of each vector cost a sector or two: there x and r
+// are updated by rows (k_tl_rows).  Us an iteration fused, and as two kernels, by the order of the
+// nodes: in order, shuffled in runs of 8, of 2, at random (gf_ctx::gather 0.06, 0.25 to 0.3, 0.6,
+// 0.8).  Up to 200k dofs the second kernel costs more than scattered sectors in L2:
+//   Q4 300^2     181k dofs  24.4, 27.7   26.0, 28.8   29.7, 30.3   37.5, 32.9
+//   Brick20 24^3 182k       63.5, 64.2   67.2, 67.7   70.5, 69.5   76.4, 72.3
+//   Brick8 40^3  207k       45.6, 46.3   49.6, 48.0   53.4, 50.8   59.2, 52.4
+//   Brick8 64^3  824k       128.8, 127.6 133.8, 131.0 150.7, 136.1 172.4, 141.2
+//   Q8 400^2     963k       89.0, 90.7   96.0, 94.7   117.7, 100.1 148.1, 107.6
 constexpr int kUT = 128, kMaxShares = 64;
-template <int DIM, bool INIT, typename V>
+template <int DIM, bool INIT, bool FUSED, typename V>
 __global__ void __launch_bounds__(kUT, 1)
 k_tl_update(const int4* __restrict__ blk, const int32_t* __restrict__ nodes,
             const double* __restrict__ xc, const double* __restrict__ cen, double sinv,
@@ -1006,15 +1029,8 @@ k_tl_update(const int4* __restrict__ blk, const int32_t* __restrict__ nodes,
   __shared__ double ws[kUT / 32][8];
   const int4 share = __ldg(blk + blockIdx.x);   // on its way while the scalars are looked at
   double alpha = 0.0;
-  if (!INIT) {
-    if (sc->done) return;
-    const double pq = sc->pq;
-    if (!(pq > 0.0) || !isfinite(pq)) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) sc->done = 2;
-      return;
-    }
-    alpha = sc->rz / pq;
-  }
+  if (!FUSED && sc->done) return;
+  if (FUSED && !INIT && !tl_alpha(sc, alpha)) return;
   const int A = share.x, row = share.w & 255, stride = (share.w >> 8) * kUT;
   double cA[DIM];
 #pragma unroll
@@ -1030,6 +1046,10 @@ k_tl_update(const int4* __restrict__ blk, const int32_t* __restrict__ nodes,
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
       d[c] = (xc[i + c] - cA[c]) * sinv;
+      if (!FUSED) {
+        ri[c] = r[i + c];
+        continue;
+      }
       f[c] = (double)dinv[i + c];
       if (INIT) {
         ri[c] = (V)(b[i + c] * scale);
@@ -1043,8 +1063,10 @@ k_tl_update(const int4* __restrict__ blk, const int32_t* __restrict__ nodes,
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
       const double rd = (double)ri[c];
-      acc[NM] += rd * rd;
-      acc[NM + 1] += rd * rd * f[c];
+      if (FUSED) {
+        acc[NM] += rd * rd;
+        acc[NM + 1] += rd * rd * f[c];
+      }
       if (fixed[i + c]) continue;
       double pr[NM];
       p_row<DIM>(c, d, pr);
@@ -1064,10 +1086,40 @@ k_tl_update(const int4* __restrict__ blk, const int32_t* __restrict__ nodes,
     if (m < NM) {
       rc[(int64_t)row * ld + A * NM + m] = u;
       if (row == 0) zc[A * NM + m] = 0.0;
-    } else {
+    } else if (FUSED) {
       atomicAdd(m == NM ? &sc->rr : &sc->rzn, u);
     }
   }
+}
+
+// The update of x and r and its sums by rows, without the restriction.
+template <bool INIT, typename V>
+__global__ void __launch_bounds__(kCT)
+k_tl_rows(int n, const double* __restrict__ b, const V* __restrict__ q, double scale,
+          V* __restrict__ x, V* __restrict__ r, const V* __restrict__ p,
+          const V* __restrict__ dinv, SolveScalars* sc) {
+  __shared__ double sh[32];
+  double alpha = 0.0;
+  if (!INIT && !tl_alpha(sc, alpha)) return;
+  double rr = 0.0, rdr = 0.0;
+  for (int i = blockIdx.x * kCT + threadIdx.x; i < n; i += gridDim.x * kCT) {
+    V ri;
+    if (INIT) {
+      ri = (V)(b[i] * scale);
+      x[i] = V(0);
+    } else {
+      x[i] += (V)alpha * p[i];
+      ri = r[i] - (V)alpha * q[i];
+    }
+    r[i] = ri;
+    const double rd = (double)ri;
+    rr += rd * rd;
+    rdr += rd * rd * (double)dinv[i];
+  }
+  const double s1 = cg_block_sum(rr, sh);
+  if (threadIdx.x == 0) atomicAdd(&sc->rr, s1);
+  const double s2 = cg_block_sum(rdr, sh);
+  if (threadIdx.x == 0) atomicAdd(&sc->rzn, s2);
 }
 
 // z = D^-1 r + P zc on the fly.  MODE kTlFirst: p = z; kTlKeep: p = pscale p (a
@@ -1287,6 +1339,7 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
   // blocks of the fused update: a thread per node while there are no more than 16 blocks per SM
   // (more start a second wave), an aggregate of up to 3/2 of the mean size as one of the mean,
   // at most kMaxShares to an aggregate; the first blocks of all aggregates, then the second ones
+  C->fused = ctx->gather <= (ctx->n <= 200000 ? 0.7f : 0.25f);
   const int mean = gf_blocks(nnodes, na);
   C->parts = std::max(1, std::min(gf_blocks(mean, kUT), 16 * ctx->sm_count / na));
   const int most = std::max(kUT, gf_blocks((int64_t)mean * 3, 2 * C->parts));
@@ -1448,14 +1501,19 @@ static void tl_launch(gf_ctx* ctx, int mode, const double* b, const V* q, double
   const int grid = std::min(gf_blocks(nn, kCT), ctx->sm_count * 8);
   const uint8_t* fx = ctx->d_fixed;
   const double* xc = ctx->d_coords64;
-  if (mode == kTlStep)
-    k_tl_update<DIM, false, V><<<c->nblk, kUT, 0, s>>>(c->blk, c->agg_nodes, xc, c->cen, sinv, fx,
-                                                       nullptr, q, 1.0, x, r, p, dinv, c->rc, ld,
-                                                       c->zc, sc);
-  else
-    k_tl_update<DIM, true, V><<<c->nblk, kUT, 0, s>>>(c->blk, c->agg_nodes, xc, c->cen, sinv, fx, b,
-                                                      nullptr, scale, x, r, nullptr, dinv, c->rc, ld,
-                                                 c->zc, sc);
+  const bool step = mode == kTlStep;
+  const V *qs = step ? q : nullptr, *ps = step ? p : nullptr;
+  if (!c->fused) {
+    auto* rows = step ? k_tl_rows<false, V> : k_tl_rows<true, V>;
+    rows<<<std::min(gf_blocks(ctx->n, kCT), ctx->sm_count * 8), kCT, 0, s>>>(ctx->n, b, qs, scale, x, r,
+                                                                            ps, dinv, sc);
+    ctx->launches++;
+  }
+  auto* update = !c->fused ? k_tl_update<DIM, false, false, V>
+                 : step    ? k_tl_update<DIM, false, true, V>
+                           : k_tl_update<DIM, true, true, V>;
+  update<<<c->nblk, kUT, 0, s>>>(c->blk, c->agg_nodes, xc, c->cen, sinv, fx, b, qs, scale, x, r, ps,
+                                 dinv, c->rc, ld, c->zc, sc);
   k_coarse_symv<<<c->ntiles, 256, 0, s>>>(c->tile_ij, c->ainv, c->rc, c->parts, c->shares, ld,
                                           c->zc, sc, &sc->done);
   auto* direction = mode == kTlFirst  ? k_tl_direction<DIM, kTlFirst, V>
