@@ -545,8 +545,9 @@ GF_API gf_status gf_assemble(gf_ctx* ctx, int32_t dtype, int32_t scatter, int32_
   if (!ctx->has_pattern && (st = gf_pattern_build(ctx)) != GF_OK) return st;
   // the fastest measured schedule (B200): Brick8 128^3 FP32 1.56 ms by owners, 3.82 ms with
   // atomics; Brick20 64^3 FP32 2.96 ms with atomics, 7.94 ms by owners
-  // small FP64 Brick8 meshes: an SM gets two warps of owners or fewer, each a serial chain of
-  // FP64 sums, 42 us at 8^3 and 48 at 21^3 against 27 and 46 with atomics (22^3: 48 and 57)
+  // small FP64 Brick8 meshes: an SM gets three warps of owners or fewer (28 nodes each), each a
+  // serial chain of FP64 sums, 42 us at 8^3 and 48 at 21^3 against 27 and 46 with atomics (22^3:
+  // 48 and 57)
   const bool b8_small = ctx->elem_type == GF_BRICK8 && dtype == GF_F64 &&
                         ctx->nnodes <= 76 * (int64_t)ctx->sm_count;
   const bool automatic = scatter == GF_SCATTER_AUTO;

@@ -1348,12 +1348,11 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
   };
   const int rows = std::max(C->parts, shares(maxcnt));
   std::vector<int4> hblk;
-  std::vector<uint8_t> hshares(ld, 0);
+  hblk.reserve((size_t)na * C->parts * 2);
   for (int y = 0; y < rows; ++y)
     for (int A = 0; A < na; ++A) {
       const int p = shares(hoff[A + 1] - hoff[A]);
       if (y < p) hblk.push_back(make_int4(A, hoff[A] + y * kUT, hoff[A + 1], y | p << 8));
-      if (y == 0) std::fill_n(hshares.begin() + A * nm, nm, (uint8_t)p);
     }
   C->nblk = (int)hblk.size();
   if ((st = gf_palloc(ctx, &C->blk, hblk.size())) != GF_OK ||
@@ -1364,8 +1363,13 @@ gf_status build(gf_ctx* ctx, Coarse* C, int target) {
   }
   GF_CUDA(ctx, cudaMemcpyAsync(C->blk, hblk.data(), sizeof(int4) * hblk.size(),
                                cudaMemcpyHostToDevice, s));
-  if (C->shares)
+  std::vector<uint8_t> hshares;
+  if (C->shares) {
+    hshares.resize(ld, 0);
+    for (int A = 0; A < na; ++A)
+      std::fill_n(hshares.begin() + A * nm, nm, (uint8_t)shares(hoff[A + 1] - hoff[A]));
     GF_CUDA(ctx, cudaMemcpyAsync(C->shares, hshares.data(), (size_t)ld, cudaMemcpyHostToDevice, s));
+  }
   const int per = (int)((maxcnt + (int64_t)kCMT * 65535 - 1) / ((int64_t)kCMT * 65535));
   const dim3 gcm(na, (maxcnt + kCMT * per - 1) / (kCMT * per));
   if (ctx->d_adj && ctx->d_adj_off && na < (1 << 24) && gf_sell_prepare(ctx, GF_F64) == GF_OK &&
